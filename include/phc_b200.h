@@ -37,7 +37,9 @@ int phc_abi_version(void);
  * counterpart in the reference, whose launch shapes are fixed at compile
  * time or passed per call.
  *   knob 0: polynomials (warps) per CTA of phc_system_evaldiff, 1..8
- *           (the rule: min(dim, 8), fewer when the scratch needs it);
+ *           (the rule: min(dim, 8), fewer when the scratch needs it; a
+ *           batch of at most 1184 polynomials takes a CTA per polynomial
+ *           instead, its monomials shared by the warps);
  *   knob 1: variant of the split tracker's kernel, 1 the 64-register one
  *           (8 paths per SM), 2 the 72-register one (7 paths per SM) (the
  *           rule: 2 when the batch fits in one wave at 7 per SM);
@@ -69,9 +71,8 @@ int phc_tune_get(int knob);
  * output: nsys*dim*(dim+1) series; polynomial (s,p) occupies dim+1 series,
  *         series j < dim the derivative with respect to x_j, series dim the
  *         value (the reference's output[dim] convention).
- * Limit: deg <= 191 (the reference's largest degree); series of up to 32
- * coefficients take one warp per product, longer ones a lane per
- * coefficient (k, k + 32, ...). */
+ * Limit: deg <= 191 (the reference's largest degree).  A warp forms a
+ * product of series, in one round up to 32 coefficients, in more beyond. */
 int phc_system_evaldiff(int prec, int cplx, int nsys, int dim, int deg, int maxvar, const int *mon_off,
                         const int *nvr, const int *idx, const int *exps, const double *cst, const double *cff,
                         const double *input, double *output, void *stream);

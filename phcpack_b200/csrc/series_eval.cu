@@ -2,11 +2,21 @@
 // systems at truncated power series (the Polynomials layer of PHCpack's GPU
 // code, Polynomials/dbl2_polynomials_kernels.cu:1577, batched over systems).
 //
-// Grid: one CTA per (system, group of up to 8 polynomials); one warp per
-// polynomial.  The CTA stages the system's input series in shared memory
-// (coalesced 16-byte loads), each warp keeps its monomial's forward and
-// backward products in its own shared-memory slots and accumulates the
+// Two arrangements.  A warp per polynomial: one CTA per (system, group of up
+// to 8 polynomials); the CTA stages the system's input series in shared
+// memory (coalesced 16-byte loads), each warp keeps its monomial's forward
+// and backward products in its own shared-memory slots and accumulates the
 // polynomial's value and gradient rows in the output buffer, which it owns.
+// A CTA per polynomial, for few polynomials: the warps share its monomials
+// and the rows are summed in shared memory in the monomials' order.
+//
+// Bound by the FP64 pipe and the latency of its operations.  1024 systems
+// (n = 32, 32 monomials, degree 31, complex double-double): 37.4 ms with the
+// multiple-double operators, 29.9 with open accumulators (md::macc), 28.5
+// with two-variable monomials in three products instead of four, 24.2 with
+// one inlined product per kernel in chunks of three terms: 70 % of the FP64
+// pipe's rate.  At 16 warps per SM; 24 (80 registers) measured 4 % slower, 8
+// with 153 registers 25 %.
 #include "common.cuh"
 #include "series_eval.cuh"
 
@@ -14,95 +24,113 @@ namespace phc {
 
 static const int kMaxWarpsPerBlock = 8;
 static const int kMaxSmem = 227 * 1024;
+// Polynomials up to which a CTA takes one: 8 warps each, so that one wave of
+// CTAs still gives every SM 8 polynomials.  One system of 8 polynomials of 12
+// monomials (degree 15, complex double-double): 68 us shared, 332 with a warp
+// per polynomial; 512 polynomials at degree 95: 1.04 ms against 2.7.
+static const long kSplitPolys = 148 * 8;
 
-template <class N>
-__global__ void __launch_bounds__(kMaxWarpsPerBlock * 32)
+// Input series of a system, n doubles, into shared memory.
+__device__ __forceinline__ void stage_inputs(const double *__restrict__ xin, double *Xs, int n) {
+  if ((n & 1) == 0 && (reinterpret_cast<unsigned long long>(xin) & 15) == 0) {
+    const double2 *src = reinterpret_cast<const double2 *>(xin);
+    double2 *dst = reinterpret_cast<double2 *>(Xs);
+    for (int i = threadIdx.x; i < n / 2; i += blockDim.x) dst[i] = src[i];
+  } else {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) Xs[i] = xin[i];
+  }
+}
+
+// A warp per polynomial.  BIG (degrees 32..191): one more scratch series per
+// warp (the value); the inputs are staged in shared memory when they fit
+// beside the scratch and read from global memory otherwise.
+template <class N, bool BIG>
+__global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, N::width <= 4 ? 2 : 1)
     k_system_evaldiff(int dim, int deg, int maxvar, int wpb, int stage, const int *__restrict__ mon_off,
                       const int *__restrict__ nvr, const int *__restrict__ idx, const int *__restrict__ exps,
                       const double *__restrict__ cst, const double *__restrict__ cff,
                       const double *__restrict__ input, double *__restrict__ output) {
   extern __shared__ __align__(16) double sm[];
-  const int W = N::width;
-  const int S = (deg + 1) * W;
+  const int S = (deg + 1) * N::width;
   const int bps = (dim + wpb - 1) / wpb;
   const int s = blockIdx.x / bps;
   const int p0 = (blockIdx.x % bps) * wpb;
-  const double *xin = input + (long)s * dim * S;
-  const double *X = xin;
+  const double *X = input + (long)s * dim * S;
   double *scr = sm;
   if (stage) {
-    double *Xs = sm;
-    const int n = dim * S;
-    if ((W & 1) == 0) {
-      const double2 *src = reinterpret_cast<const double2 *>(xin);
-      double2 *dst = reinterpret_cast<double2 *>(Xs);
-      for (int i = threadIdx.x; i < n / 2; i += blockDim.x) dst[i] = src[i];
-    } else {
-      for (int i = threadIdx.x; i < n; i += blockDim.x) Xs[i] = xin[i];
-    }
-    X = Xs;
-    scr = sm + ((n + 1) & ~1);
+    stage_inputs(X, sm, dim * S);
+    X = sm;
+    scr = sm + ((dim * S + 1) & ~1);
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5;
   const int p = p0 + warp;
   if (p >= dim) return;
-  scr += (long)warp * warp_slots(maxvar) * S;
+  scr += (long)warp * (warp_slots(maxvar) + (BIG ? 1 : 0)) * S;
   const long sp = (long)s * dim + p;
-  warp_poly_evaldiff<N>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, cst + sp * S, cff, X, scr,
-                        output + sp * (dim + 1) * S);
+  warp_poly_evaldiff<N, BIG>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, cst + sp * S, cff, X,
+                             scr, output + sp * (dim + 1) * S);
 }
 
-// Degrees 32..191: the same grid, warp_poly_evaldiff_big, one more scratch
-// series per warp (the value); the inputs are staged in shared memory when
-// they fit beside the scratch and read from global memory otherwise.
-template <class N>
-__global__ void __launch_bounds__(kMaxWarpsPerBlock * 32)
-    k_system_evaldiff_big(int dim, int deg, int maxvar, int wpb, int stage, const int *__restrict__ mon_off,
-                          const int *__restrict__ nvr, const int *__restrict__ idx, const int *__restrict__ exps,
-                          const double *__restrict__ cst, const double *__restrict__ cff,
-                          const double *__restrict__ input, double *__restrict__ output) {
+// A CTA per polynomial, its monomials shared by the warps.
+template <class N, bool BIG>
+__global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, N::width <= 4 ? 2 : 1)
+    k_poly_evaldiff(int dim, int deg, int maxvar, int stage, const int *__restrict__ mon_off,
+                    const int *__restrict__ nvr, const int *__restrict__ idx, const int *__restrict__ exps,
+                    const double *__restrict__ cst, const double *__restrict__ cff, const double *__restrict__ input,
+                    double *__restrict__ output) {
   extern __shared__ __align__(16) double sm[];
-  const int W = N::width;
-  const int S = (deg + 1) * W;
-  const int bps = (dim + wpb - 1) / wpb;
-  const int s = blockIdx.x / bps;
-  const int p0 = (blockIdx.x % bps) * wpb;
-  const double *xin = input + (long)s * dim * S;
-  const double *X = xin;
-  double *scr = sm;
+  const int S = (deg + 1) * N::width;
+  const long sp = blockIdx.x;
+  const double *X = input + (sp / dim) * dim * S;
+  double *rows = sm;
+  double *scr = sm + (((dim + 1) * S + 1) & ~1);
   if (stage) {
-    double *Xs = sm;
-    const int n = dim * S;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) Xs[i] = xin[i];
-    X = Xs;
-    scr = sm + ((n + 1) & ~1);
+    stage_inputs(X, scr, dim * S);
+    X = scr;
+    scr += (dim * S + 1) & ~1;
   }
   __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  const int p = p0 + warp;
-  if (p >= dim) return;
-  scr += (long)warp * (warp_slots(maxvar) + 1) * S;
-  const long sp = (long)s * dim + p;
-  warp_poly_evaldiff_big<N>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, cst + sp * S, cff, X,
-                            scr, output + sp * (dim + 1) * S);
+  cta_poly_evaldiff<N, BIG>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, cst + sp * S, cff, X,
+                            scr, rows, output + sp * (dim + 1) * S);
 }
 
 template <class N>
 static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_off, const int *nvr, const int *idx,
                          const int *exps, const double *cst, const double *cff, const double *input, double *output,
                          cudaStream_t stream) {
-  const int W = N::width;
-  const int S = (deg + 1) * W;
-  const bool big = deg > 31;  // series longer than a warp: k_system_evaldiff_big
+  const int S = (deg + 1) * N::width;
+  const bool big = deg > 31;  // series longer than a warp
+  const long series = (long)S * sizeof(double);
+  const long xs = (long)((dim * S + 1) & ~1) * sizeof(double);
+  const int tuned = tune_get(kTuneEvalWarps);  // warps per CTA chosen by the autotuner
+  // A warp per polynomial leaves most of the GPU idle on a few systems, and
+  // each warp's products follow one another.  While the polynomials are
+  // fewer than kSplitPolys a CTA takes one polynomial and shares its
+  // monomials among its warps, when the rows fit in shared memory.
+  if (tuned == 0 && (long)nsys * dim <= kSplitPolys) {
+    const long per_warp = (warp_slots(maxvar) + maxvar + 1) * series;
+    const long rows = (long)(((dim + 1) * S + 1) & ~1) * sizeof(double);
+    int nw = kMaxWarpsPerBlock;
+    while (nw > 2 && rows + nw * per_warp > kMaxSmem - 1024) --nw;
+    long smem = rows + nw * per_warp;
+    if (smem <= kMaxSmem - 1024) {
+      const int stage = smem + xs <= 200 * 1024;
+      if (stage) smem += xs;
+      auto kern = big ? k_poly_evaldiff<N, true> : k_poly_evaldiff<N, false>;
+      PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<(unsigned)(nsys * dim), nw * 32, smem, stream>>>(dim, deg, maxvar, stage, mon_off, nvr, idx, exps, cst,
+                                                               cff, input, output);
+      PHC_CHECK_LAUNCH();
+      return PHC_OK;
+    }
+  }
   // one warp per polynomial, up to 8 per CTA; monomials with many variables
   // need many scratch series per warp, so fewer warps share a CTA when the
   // shared memory would not hold the scratch of 8; the inputs are staged in
   // shared memory when they fit beside the scratch
-  const long per_warp = (long)(warp_slots(maxvar) + (big ? 1 : 0)) * S * sizeof(double);
-  const long xs = (long)((dim * S + 1) & ~1) * sizeof(double);
+  const long per_warp = (warp_slots(maxvar) + (big ? 1 : 0)) * series;
   int wpb = dim < kMaxWarpsPerBlock ? dim : kMaxWarpsPerBlock;
-  const int tuned = tune_get(kTuneEvalWarps);  // warps per CTA chosen by the autotuner
   if (tuned > 0) wpb = tuned < dim ? tuned : dim;
   while (wpb > 1 && (long)wpb * per_warp > kMaxSmem) --wpb;
   const long scr = (long)wpb * per_warp;
@@ -112,7 +140,7 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
     set_error("system_evaldiff: %ld bytes of shared memory needed (maxvar %d, degree %d)", smem, maxvar, deg);
     return PHC_ERR_LIMIT;
   }
-  auto kern = big ? k_system_evaldiff_big<N> : k_system_evaldiff<N>;
+  auto kern = big ? k_system_evaldiff<N, true> : k_system_evaldiff<N, false>;
   PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int bps = (dim + wpb - 1) / wpb;
   const long grid = (long)nsys * bps;

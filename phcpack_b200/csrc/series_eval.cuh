@@ -7,108 +7,129 @@
 // thread k does k+1 of the d+1 padded steps.  Here one warp computes one
 // product: coefficients k and d-k are paired (together d+2 terms), and the
 // two lanes of a pair split those terms in halves, so every lane does
-// ceil((d+2)/2) steps; one shuffle exchange adds the halves.  Series live
-// in shared memory, limb-interleaved.
+// ceil((d+2)/2) steps; one shuffle exchange adds the halves.  A warp holds 16
+// pairs: series of up to 32 coefficients take one round, longer ones
+// ceil((d+1)/32) rounds of the same number of steps.  Series live in shared
+// memory, limb-interleaved.
 #pragma once
 #include "md.cuh"
 
 namespace phc {
 
-// lane mapping of a degree-deg product, deg+1 <= 32
+// Lane mapping of round r of a degree-deg product: lane 16 h + l is half h of
+// pair p = 16 r + l.  Every lane does nch chunks of U terms.  Half 0 does
+// the k1 + 1 terms of k1 in its first sw chunks, then the first cnt2 terms of
+// k2; half 1 the rest of k2 from x_i0 y_j0 on.  (Chunks, so that a lane turns
+// from k1 to k2 between straight-line blocks of U products; the last chunk
+// of a part may be short.)  A middle coefficient (k1 = k2, even degree) is
+// shared like a k2.
+template <int U>
 struct lanemap {
-  int p, h, k1, k2, t0, t1, partner, steps;
+  int k1, k2, i0, j0, cnt, cnt2, sw, nch, h;
+  bool alone;  // half 0 of a pair: its own coefficient k1 needs nothing from the other half
   bool valid;  // this lane owns output coefficient kout()
-  __device__ __forceinline__ lanemap(int deg, int lane) {
-    const int n1 = deg + 1;
-    const int np = (n1 + 1) >> 1;
-    const bool active = lane < 2 * np;
-    p = active ? lane % np : 0;
-    h = active ? lane / np : 0;
+  __device__ __forceinline__ lanemap(int deg, int lane, int round) {
+    const int np = (deg + 2) >> 1;
+    const int pp = 16 * round + (lane & 15);
+    const bool active = pp < np;
+    const int p = active ? pp : 0;
+    h = lane >> 4;
     k1 = p;
     k2 = deg - p;
-    const int nt = (k1 == k2) ? (p + 1) : (deg + 2);
-    const int half = (nt + 1) >> 1;
-    t0 = (h == 0) ? 0 : half;
-    t1 = (h == 0) ? half : nt;
-    if (!active) t0 = t1 = 0;
-    partner = active ? (h == 0 ? lane + np : lane - np) : lane;
-    steps = ((deg + 2) + 1) >> 1;
-    valid = active && !(h == 1 && k1 == k2);
+    nch = ((deg + 2 + U) / 2 + U - 1) / U;  // 2 nch U >= deg + 1 - p + a for a <= p + U
+    const bool mid = k1 == k2;
+    const int a = mid ? 0 : (p + U) / U;  // chunks of k1
+    const int n2 = k2 + 1;                // terms of k2
+    const int first = mid ? (n2 + 1) >> 1 : min((nch - a) * U, n2);
+    alone = h == 0 && !mid;
+    cnt2 = first;
+    cnt = !active ? 0 : (h == 0 ? (mid ? first : p + 1) : n2 - first);
+    sw = (active && alone) ? a : -1;
+    i0 = h == 0 ? 0 : first;
+    j0 = (alone ? k1 : k2) - i0;
+    valid = active && !(h == 1 && mid);
   }
   __device__ __forceinline__ int kout() const { return h == 0 ? k1 : k2; }
 };
 
-template <class N>
+// Terms per chunk: quad-double's products are long enough by themselves; at
+// degree 31 three take 18 terms per lane where one takes 17.
+template <class N> struct conv_chunk { static const int U = N::tr::limbs == 4 ? 1 : 3; };
+
+// Series of one warp.  BIG: longer than 32 coefficients, several rounds.
+template <class N, bool BIG>
 struct wser {
   typedef typename N::T T;
   static const int W = N::width;
+  static const int U = conv_chunk<N>::U;
+  typedef lanemap<U> map;
+  int deg, n1, lane;
+
+  __device__ __forceinline__ wser(int deg_, int lane_) : deg(deg_), n1(deg_ + 1), lane(lane_) {}
 
   // z = x*y (x, y series in shared memory); returns the coefficient this
   // lane owns (m.valid) at index m.kout().  All 32 lanes must call it.
-  // Compiled once and called (not inlined at its many call sites): the
-  // evaluation kernel is bound by instruction fetch when every call site
-  // carries its own copy of the loop.
-  static __device__ __noinline__ T conv(const double *x, const double *y, const lanemap &m) {
-    T a1 = N::zero(), a2 = N::zero();
-    for (int s = 0; s < m.steps; ++s) {
-      const int t = m.t0 + s;
-      if (t < m.t1) {
-        const bool first = (t <= m.p);
-        const int i = first ? t : t - (m.p + 1);
-        const int j = (first ? m.k1 : m.k2) - i;
-        T xi, yj;
-        md::ldn(x + i * W, xi);
-        md::ldn(y + j * W, yj);
-        const T pr = N::mul(xi, yj);
-        T a = first ? a1 : a2;
-        a = N::add(a, pr);
-        if (first) a1 = a; else a2 = a;
+  //
+  // The products go into one open accumulator (msum).  A lane of the first
+  // half sums its k1 terms first and puts that sum aside when it turns to
+  // its share of k2 (at chunk m.sw).
+  static __device__ __forceinline__ T conv(const double *x, const double *y, const map &m) {
+    md::msum<N> acc, done;
+    acc.zero();
+    done.zero();
+    const double *px = x + m.i0 * W, *py = y + m.j0 * W;
+    int left = m.cnt;
+#pragma unroll 1
+    for (int c = 0; c < m.nch; ++c) {
+      if (c == m.sw) {  // k1 is complete; on to x_0 y_k2 + ...
+        done = acc;
+        acc.zero();
+        px = x;
+        py = y + m.k2 * W;
+        left = m.cnt2;
       }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        T xi = N::zero(), yj = N::zero();
+        if (left > u) {
+          md::ldn(px + u * W, xi);
+          md::ldn(py - u * W, yj);
+        }
+        acc.fma(xi, yj);
+      }
+      px += U * W;
+      py -= U * W;
+      left -= U;
     }
-    const T o1 = md::shfl(a1, m.partner);
-    const T o2 = md::shfl(a2, m.partner);
-    return (m.h == 0) ? N::add(a1, o1) : N::add(a2, o2);
+    if (m.sw == m.nch) {
+      done = acc;
+      acc.zero();
+    }
+    const T a = acc.value();
+    const T o = md::shfl_xor(a, 16);
+    return m.alone ? done.value() : N::add(a, o);
   }
 
-  // dst[k] = z (shared memory), then make it visible to the warp
-  static __device__ __forceinline__ void put(double *dst, const T &z, const lanemap &m) {
-    if (m.valid) md::stn(dst + m.kout() * W, z);
-    __syncwarp();
-  }
-  static __device__ __forceinline__ void prod(const double *x, const double *y, double *z, const lanemap &m) {
-    const T r = conv(x, y, m);
-    __syncwarp();  // z may alias a buffer other lanes still read
-    put(z, r, m);
-  }
-  // row[k] += e*z in global memory (lane-owned coefficient); the first
-  // contribution to a row (first == true) is stored without reading it
-  static __device__ __forceinline__ void acc_global(double *row, const T &z, const lanemap &m, int e, bool first) {
-    if (m.valid) {
-      const T zz = (e > 1) ? N::scale_d(z, (double)e) : z;
-      if (first) {
-        md::stn(row + m.kout() * W, zz);
-      } else {
-        T v;
-        md::ldn(row + m.kout() * W, v);
-        md::stn(row + m.kout() * W, N::add(v, zz));
-      }
+  __device__ __forceinline__ int rounds() const { return BIG ? (n1 + 31) >> 5 : 1; }
+  // f(k) for the coefficients k, lane k mod 32
+  template <class F>
+  __device__ __forceinline__ void coefs(F f) const {
+    if constexpr (BIG) {
+#pragma unroll 1
+      for (int k = lane; k < n1; k += 32) f(k);
+    } else {
+      if (lane < n1) f(lane);
     }
   }
-  // row[k] += e*src[k] for a series src in shared memory, lane k
-  static __device__ __forceinline__ void acc_series(double *row, const double *src, int n1, int e, bool first) {
-    const int lane = threadIdx.x & 31;
-    if (lane < n1) {
-      T z;
-      md::ldn(src + lane * W, z);
-      if (e > 1) z = N::scale_d(z, (double)e);
-      if (first) {
-        md::stn(row + lane * W, z);
-      } else {
-        T v;
-        md::ldn(row + lane * W, v);
-        md::stn(row + lane * W, N::add(v, z));
-      }
-    }
+  __device__ __forceinline__ void copy(const double *src, double *dst) const {
+    coefs([&](int k) {
+      T v;
+      md::ldn(src + k * W, v);
+      md::stn(dst + k * W, v);
+    });
+  }
+  __device__ __forceinline__ void clear(double *dst) const {
+    coefs([&](int k) { md::stn(dst + k * W, N::zero()); });
   }
 };
 
@@ -119,275 +140,284 @@ __host__ __device__ inline int warp_slots(int maxvar) {
   return s < 3 ? 3 : s;
 }
 
-// Value and gradient of one polynomial of a system, accumulated by one warp
-// into out (dim+1 series in global memory; row dim is the value).  The
-// value is accumulated in registers (each lane its coefficients) and
-// written once.  A gradient row is stored at its first contribution and
-// read, added to and written back only after that (a 64-bit mask records
-// the rows 0..63 written so far; rows from 64 on are zeroed first and
-// always accumulated); rows no monomial reached are zeroed at the end.
-//
-// Per monomial: the common-factor method of Newton/dbl2_systems_host.cpp:
-// 18-110 (coefficient <- x^(e-1) * coefficient, derivative j scaled by e_j),
-// then the forward/backward/cross products of
-// Convolutions/dbl2_monomials_host.cpp:4-22 (CPU_dbl2_evaldiff, :175).
-template <class N>
-__device__ void warp_poly_evaldiff(int dim, int deg, int maxvar, int m0, int m1, const int *__restrict__ nvr,
-                                   const int *__restrict__ idx, const int *__restrict__ exps,
-                                   const double *__restrict__ cst, const double *__restrict__ cff,
-                                   const double *X,  // shared: dim series
-                                   double *scr,      // shared: warp_slots(maxvar) series
-                                   double *out) {
+// One monomial by one warp: its value and its k partial derivatives go to
+// the sink.  The common-factor method of Newton/dbl2_systems_host.cpp:18-110
+// (coefficient c <- x^(e-1) c, derivative j scaled by e_j), then the forward,
+// backward and cross products of Convolutions/dbl2_monomials_host.cpp:4-22
+// (CPU_dbl2_evaldiff, :175), 3k - 3 of them:
+//   f_j = f_{j-1} x_j (f_{-1} = c, j <= k-2; f_{k-2} is the derivative in x_{k-1});
+//   the value f_{k-2} x_{k-1};
+//   b_0 = x_{k-1} x_{k-2}, b_i = b_{i-1} x_{k-2-i} (i <= k-3);
+//   the derivative in x_0, b_{k-3} c;
+//   those in x_{i+1}: f_i b_{k-4-i} (i <= k-4) and f_{k-3} x_{k-1} (i = k-3);
+//   two variables: c x_1 is the derivative in x_0, times x_0 the value, and
+//   x_0 c the derivative in x_1.
+// All products run through one loop with one inlined copy of the series
+// product: a call per product would keep the caller's state in registers
+// across it, which the product needs for independent operations in flight
+// (FP64 latency, not the pipe, limited the evaluation), and a copy per kind
+// of product would not fit the instruction cache.
+// X: dim series (shared memory or global); scr: warp_slots(maxvar) series of
+// shared memory.  A malformed monomial (variable count, index or exponent
+// out of range) is skipped rather than read out of bounds; the host entry
+// points reject such supports before any launch.  Returns the number of
+// variables, 0 for a skipped monomial.
+template <class N, bool BIG, class Sink>
+__device__ __forceinline__ int warp_monomial(const wser<N, BIG> &ws, int dim, int maxvar, int k,
+                                             const int *__restrict__ ix, const int *__restrict__ ex,
+                                             const double *__restrict__ cffm, const double *X, double *scr,
+                                             Sink &sink) {
   typedef typename N::T T;
-  const int W = N::width;
-  const int n1 = deg + 1;
-  const int S = n1 * W;  // doubles per series
-  const int lane = threadIdx.x & 31;
-  const lanemap m(deg, lane);
-  typedef wser<N> ws;
-
-  // rows past the first 64 start at zero (the mask covers rows 0..63)
-  for (int r = 64; r < dim; ++r)
-    if (lane < n1) md::stn(out + r * S + lane * W, N::zero());
-  unsigned long long written = 0ull;  // gradient rows stored so far (uniform over the warp)
-  auto first_touch = [&](int r) {
-    if (r >= 64) return false;
-    const bool f = !((written >> r) & 1ull);
-    written |= 1ull << r;
-    return f;
-  };
-  // the value starts at the constant series, lane-owned coefficients
-  T vacc = N::zero();
-  if (m.valid) md::ldn(cst + m.kout() * W, vacc);
-  double *C = scr;
-  double *Tm = scr + S;
-  double *F = scr + 2 * S;                 // f_0 .. f_{k-2}
-  double *B = scr + (1 + maxvar) * S;      // b_0 .. b_{k-3}
-
-  for (int mon = m0; mon < m1; ++mon) {
-    const int k = nvr[mon];
-    const int *ix = idx + mon * maxvar;
-    const int *ex = exps + mon * maxvar;
-    // a malformed monomial (variable count, index or exponent out of range)
-    // is skipped rather than read out of bounds; the host entry points
-    // reject such supports before any launch
-    bool ok = (k >= 1 && k <= maxvar);
-    for (int v = 0; ok && v < k; ++v) ok = (ix[v] >= 0 && ix[v] < dim && ex[v] >= 1);
-    if (!ok) continue;
-    if (lane < n1) {
-      T c;
-      md::ldn(cff + (long)mon * S + lane * W, c);
-      md::stn(C + lane * W, c);
+  const int S = ws.n1 * N::width;
+  bool ok = (k >= 1 && k <= maxvar);
+  for (int v = 0; ok && v < k; ++v) ok = (ix[v] >= 0 && ix[v] < dim && ex[v] >= 1);
+  if (!ok) return 0;
+  double *const F = scr + 2 * S;                 // f_0 .. f_{k-2}
+  double *const B = scr + (1 + maxvar) * S;      // b_0 .. b_{k-3}
+  ws.copy(cffm, scr);
+  __syncwarp();
+  int cslot = 0;         // c is scratch series 0 or 1
+  int v = 0, r = 1;      // next common factor: the r-th of variable v
+  int j = 0;             // next of the 3k - 3 products (1 when k = 1)
+  const int nprod = k == 1 ? 1 : 3 * k - 3;
+#pragma unroll 1
+  for (;;) {
+    const double *C = scr + cslot * S;
+    const double *x, *y;
+    double *dst = nullptr;  // scratch series that takes the product
+    int var = -1;           // variable whose derivative it is
+    bool value = false;
+    while (v < k && r >= ex[v]) {
+      ++v;
+      r = 1;
     }
-    __syncwarp();
-    // common factors: C <- x_v^(e_v - 1) * C
-    for (int v = 0; v < k; ++v) {
-      const int e = ex[v];
-      for (int r = 1; r < e; ++r) {
-        ws::prod(X + ix[v] * S, C, Tm, m);
-        double *t = C; C = Tm; Tm = t;
-      }
-    }
-    if (k == 1) {
-      const T z = ws::conv(X + ix[0] * S, C, m);
-      if (m.valid) vacc = N::add(vacc, z);
-      ws::acc_series(out + ix[0] * S, C, n1, ex[0], first_touch(ix[0]));
-    } else if (k == 2) {
-      ws::prod(X + ix[0] * S, X + ix[1] * S, Tm, m);
-      T z = ws::conv(Tm, C, m);
-      if (m.valid) vacc = N::add(vacc, z);
-      z = ws::conv(C, X + ix[0] * S, m);
-      ws::acc_global(out + ix[1] * S, z, m, ex[1], first_touch(ix[1]));
-      z = ws::conv(C, X + ix[1] * S, m);
-      ws::acc_global(out + ix[0] * S, z, m, ex[0], first_touch(ix[0]));
-    } else {
-      // forward products f_i = f_{i-1} x_i, f_0 = c x_0
-      ws::prod(C, X + ix[0] * S, F, m);
-      for (int i = 1; i < k - 1; ++i) ws::prod(F + (i - 1) * S, X + ix[i] * S, F + i * S, m);
-      T z = ws::conv(F + (k - 2) * S, X + ix[k - 1] * S, m);
-      if (m.valid) vacc = N::add(vacc, z);
-      ws::acc_series(out + ix[k - 1] * S, F + (k - 2) * S, n1, ex[k - 1], first_touch(ix[k - 1]));
-      // backward products b_0 = x_{k-1} x_{k-2}, b_i = b_{i-1} x_{k-2-i}
-      ws::prod(X + ix[k - 1] * S, X + ix[k - 2] * S, B, m);
-      for (int i = 1; i < k - 2; ++i) ws::prod(B + (i - 1) * S, X + ix[k - 2 - i] * S, B + i * S, m);
-      // b_{k-3} <- b_{k-3} * c : derivative in x_0
-      z = ws::conv(B + (k - 3) * S, C, m);
-      __syncwarp();
-      ws::put(B + (k - 3) * S, z, m);
-      ws::acc_series(out + ix[0] * S, B + (k - 3) * S, n1, ex[0], first_touch(ix[0]));
-      // cross products: derivative in x_j, 1 <= j <= k-2
-      if (k == 3) {
-        z = ws::conv(F, X + ix[2] * S, m);
-        ws::acc_global(out + ix[1] * S, z, m, ex[1], first_touch(ix[1]));
+    if (v < k) {
+      x = X + ix[v] * S;
+      y = C;
+      cslot ^= 1;
+      dst = scr + cslot * S;
+      ++r;
+    } else if (j < nprod) {
+      if (j < k - 1) {
+        x = j == 0 ? C : F + (j - 1) * S;
+        y = X + ix[k == 2 ? 1 : j] * S;
+        dst = F + j * S;
+        if (j == k - 2) var = k == 2 ? 0 : k - 1;
+      } else if (j == k - 1) {
+        x = k == 1 ? C : F + (k - 2) * S;
+        y = X + ix[k == 2 ? 0 : k - 1] * S;
+        value = true;
+      } else if (j < 2 * k - 2) {
+        const int i = j - k;
+        x = i == 0 ? X + ix[k - 1] * S : B + (i - 1) * S;
+        y = X + ix[k - 2 - i] * S;
+        dst = B + i * S;
+      } else if (j == 2 * k - 2) {
+        x = k == 2 ? X + ix[0] * S : B + (k - 3) * S;
+        y = C;
+        var = k == 2 ? 1 : 0;
       } else {
-        for (int i = 0; i < k - 3; ++i) {
-          z = ws::conv(F + i * S, B + (k - 4 - i) * S, m);
-          ws::acc_global(out + ix[i + 1] * S, z, m, ex[i + 1], first_touch(ix[i + 1]));
-        }
-        z = ws::conv(F + (k - 3) * S, X + ix[k - 1] * S, m);
-        ws::acc_global(out + ix[k - 2] * S, z, m, ex[k - 2], first_touch(ix[k - 2]));
+        const int i = j - (2 * k - 1);
+        x = F + i * S;
+        y = i == k - 3 ? X + ix[k - 1] * S : B + (k - 4 - i) * S;
+        var = i + 1;
+      }
+      ++j;
+    } else {
+      break;
+    }
+    const bool deriv = var >= 0;
+    const int row = deriv ? ix[var] : 0, e = deriv ? ex[var] : 1;
+    if (deriv) sink.open(row);
+#pragma unroll 1
+    for (int q = 0; q < ws.rounds(); ++q) {
+      const typename wser<N, BIG>::map m(ws.deg, ws.lane, q);
+      const T z = wser<N, BIG>::conv(x, y, m);
+      if (m.valid) {
+        const int kk = m.kout();
+        if (dst) md::stn(dst + kk * N::width, z);
+        if (value) sink.value(kk, z);
+        if (deriv) sink.derivative(var, row, e, kk, z);
       }
     }
     __syncwarp();
   }
-  // the value, and zeros in the rows no monomial reached
-  if (m.valid) md::stn(out + dim * S + m.kout() * W, vacc);
-  for (int r = 0; r < dim && r < 64; ++r)
-    if (!((written >> r) & 1ull) && lane < n1) md::stn(out + r * S + lane * W, N::zero());
-}
-
-// ------------------------------------------------------- degrees 32..191
-// Series longer than a warp: each lane owns the coefficients k = lane,
-// lane + 32, ... of a product, each formed in the reference's order
-// x_0 y_k + x_1 y_{k-1} + ... + x_k y_0 (CPU_dbl2_product,
-// Convolutions/dbl2_convolutions_host.cpp:7); the lanes of a 32-coefficient
-// chunk differ by at most 32 terms.  Compiled once and called.
-template <class N>
-__device__ __noinline__ typename N::T conv_at(const double *x, const double *y, int k) {
-  typedef typename N::T T;
-  const int W = N::width;
-  T a = N::zero();
-  for (int i = 0; i <= k; ++i) {
-    T xi, yj;
-    md::ldn(x + i * W, xi);
-    md::ldn(y + (k - i) * W, yj);
-    a = N::add(a, N::mul(xi, yj));
+  if (k == 1) {  // the derivative is c itself
+    const double *C = scr + cslot * S;
+    sink.open(ix[0]);
+    ws.coefs([&](int kk) {
+      T z;
+      md::ldn(C + kk * N::width, z);
+      sink.derivative(0, ix[0], ex[0], kk, z);
+    });
+    __syncwarp();
   }
-  return a;
+  return k;
 }
 
-// warp_poly_evaldiff for deg + 1 > 32 coefficients: the same monomial
-// method and the same outputs; the value accumulates in a series of the
-// warp's scratch (slot warp_slots(maxvar)), the products go through the
-// scratch coefficient by coefficient.
-template <class N>
-__device__ void warp_poly_evaldiff_big(int dim, int deg, int maxvar, int m0, int m1, const int *__restrict__ nvr,
-                                       const int *__restrict__ idx, const int *__restrict__ exps,
-                                       const double *__restrict__ cst, const double *__restrict__ cff,
-                                       const double *X,  // dim series (shared memory or global)
-                                       double *scr,      // shared: warp_slots(maxvar) + 1 series
-                                       double *out) {
+// Sink of a warp that owns a polynomial: value and gradient accumulate in
+// out (dim+1 series in global memory; row dim is the value).  The value of a
+// short series is kept in registers (each lane its coefficient), that of a
+// long one in the scratch series Vs, and written once.  A gradient row is
+// stored at its first contribution and read, added to and written back only
+// after that (a 64-bit mask records the rows 0..63 written so far; rows from
+// 64 on are zeroed first and always accumulated).
+template <class N, bool BIG>
+struct row_sink {
   typedef typename N::T T;
-  const int W = N::width;
-  const int n1 = deg + 1;
-  const int S = n1 * W;
-  const int lane = threadIdx.x & 31;
-  for (int r = 64; r < dim; ++r)
-    for (int k = lane; k < n1; k += 32) md::stn(out + r * S + k * W, N::zero());
-  unsigned long long written = 0ull;
-  auto first_touch = [&](int r) {
+  static const int W = N::width;
+  const wser<N, BIG> &ws;
+  double *out, *Vs;
+  unsigned long long written;
+  bool first;
+  T vacc;
+  __device__ __forceinline__ row_sink(const wser<N, BIG> &w, double *o, double *vs, int dim, const double *cst)
+      : ws(w), out(o), Vs(vs), written(0ull), first(false) {
+    vacc = N::zero();
+    for (int r = 64; r < dim; ++r) ws.clear(out + (long)r * ws.n1 * W);
+    // the value starts at the constant series
+    if constexpr (BIG) {
+      ws.copy(cst, Vs);
+      __syncwarp();
+    } else {
+      const typename wser<N, BIG>::map m(ws.deg, ws.lane, 0);
+      if (m.valid) md::ldn(cst + m.kout() * W, vacc);
+    }
+  }
+  __device__ __forceinline__ bool first_touch(int r) {
     if (r >= 64) return false;
     const bool f = !((written >> r) & 1ull);
     written |= 1ull << r;
     return f;
-  };
-  double *C = scr;
-  double *Tm = scr + S;
-  double *F = scr + 2 * S;                 // f_0 .. f_{k-2}
-  double *B = scr + (1 + maxvar) * S;      // b_0 .. b_{k-3}
-  double *Vs = scr + warp_slots(maxvar) * S;  // the value
-  for (int k = lane; k < n1; k += 32) {
-    T c;
-    md::ldn(cst + k * W, c);
-    md::stn(Vs + k * W, c);
   }
-  // z = x y into the scratch series z (z is neither x nor y)
-  auto prod = [&](const double *x, const double *y, double *z) {
-    for (int k = lane; k < n1; k += 32) md::stn(z + k * W, conv_at<N>(x, y, k));
-    __syncwarp();
-  };
-  auto add_value = [&](const double *x, const double *y) {
-    for (int k = lane; k < n1; k += 32) {
-      const T z = conv_at<N>(x, y, k);
+  __device__ __forceinline__ void value(int k, const T &z) {
+    if constexpr (BIG) {
       T v;
       md::ldn(Vs + k * W, v);
       md::stn(Vs + k * W, N::add(v, z));
-    }
-  };
-  // row += e x y (global memory; the first contribution is stored)
-  auto acc_prod = [&](double *row, const double *x, const double *y, int e, bool first) {
-    for (int k = lane; k < n1; k += 32) {
-      T z = conv_at<N>(x, y, k);
-      if (e > 1) z = N::scale_d(z, (double)e);
-      if (first) {
-        md::stn(row + k * W, z);
-      } else {
-        T v;
-        md::ldn(row + k * W, v);
-        md::stn(row + k * W, N::add(v, z));
-      }
-    }
-  };
-  // row += e src (src a scratch series)
-  auto acc_src = [&](double *row, const double *src, int e, bool first) {
-    for (int k = lane; k < n1; k += 32) {
-      T z;
-      md::ldn(src + k * W, z);
-      if (e > 1) z = N::scale_d(z, (double)e);
-      if (first) {
-        md::stn(row + k * W, z);
-      } else {
-        T v;
-        md::ldn(row + k * W, v);
-        md::stn(row + k * W, N::add(v, z));
-      }
-    }
-  };
-
-  for (int mon = m0; mon < m1; ++mon) {
-    const int k = nvr[mon];
-    const int *ix = idx + mon * maxvar;
-    const int *ex = exps + mon * maxvar;
-    bool ok = (k >= 1 && k <= maxvar);
-    for (int v = 0; ok && v < k; ++v) ok = (ix[v] >= 0 && ix[v] < dim && ex[v] >= 1);
-    if (!ok) continue;
-    for (int c = lane; c < n1; c += 32) {
-      T v;
-      md::ldn(cff + (long)mon * S + c * W, v);
-      md::stn(C + c * W, v);
-    }
-    __syncwarp();
-    // common factors: C <- x_v^(e_v - 1) * C
-    for (int v = 0; v < k; ++v)
-      for (int r = 1; r < ex[v]; ++r) {
-        prod(X + ix[v] * S, C, Tm);
-        double *t = C; C = Tm; Tm = t;
-      }
-    if (k == 1) {
-      add_value(X + ix[0] * S, C);
-      acc_src(out + ix[0] * S, C, ex[0], first_touch(ix[0]));
-    } else if (k == 2) {
-      prod(X + ix[0] * S, X + ix[1] * S, Tm);
-      add_value(Tm, C);
-      acc_prod(out + ix[1] * S, C, X + ix[0] * S, ex[1], first_touch(ix[1]));
-      acc_prod(out + ix[0] * S, C, X + ix[1] * S, ex[0], first_touch(ix[0]));
     } else {
-      prod(C, X + ix[0] * S, F);
-      for (int i = 1; i < k - 1; ++i) prod(F + (i - 1) * S, X + ix[i] * S, F + i * S);
-      add_value(F + (k - 2) * S, X + ix[k - 1] * S);
-      acc_src(out + ix[k - 1] * S, F + (k - 2) * S, ex[k - 1], first_touch(ix[k - 1]));
-      prod(X + ix[k - 1] * S, X + ix[k - 2] * S, B);
-      for (int i = 1; i < k - 2; ++i) prod(B + (i - 1) * S, X + ix[k - 2 - i] * S, B + i * S);
-      prod(B + (k - 3) * S, C, Tm);  // b_{k-3} c: the derivative in x_0
-      acc_src(out + ix[0] * S, Tm, ex[0], first_touch(ix[0]));
-      if (k == 3) {
-        acc_prod(out + ix[1] * S, F, X + ix[2] * S, ex[1], first_touch(ix[1]));
-      } else {
-        for (int i = 0; i < k - 3; ++i)
-          acc_prod(out + ix[i + 1] * S, F + i * S, B + (k - 4 - i) * S, ex[i + 1], first_touch(ix[i + 1]));
-        acc_prod(out + ix[k - 2] * S, F + (k - 3) * S, X + ix[k - 1] * S, ex[k - 2], first_touch(ix[k - 2]));
+      vacc = N::add(vacc, z);
+    }
+  }
+  // a monomial is about to contribute to gradient row r
+  __device__ __forceinline__ void open(int r) { first = first_touch(r); }
+  // row[k] += e z, stored when it is the row's first contribution
+  __device__ __forceinline__ void derivative(int, int r, int e, int k, const T &z) {
+    double *row = out + ((long)r * ws.n1 + k) * W;
+    T v = (e > 1) ? N::scale_d(z, (double)e) : z;
+    if (!first) {
+      T o;
+      md::ldn(row, o);
+      v = N::add(o, v);
+    }
+    md::stn(row, v);
+  }
+  // the value, and zeros in the rows no monomial reached
+  __device__ __forceinline__ void finish(int dim) {
+    double *row = out + (long)dim * ws.n1 * W;
+    if constexpr (BIG) {
+      ws.copy(Vs, row);
+    } else {
+      const typename wser<N, BIG>::map m(ws.deg, ws.lane, 0);
+      if (m.valid) md::stn(row + m.kout() * W, vacc);
+    }
+    for (int r = 0; r < dim && r < 64; ++r)
+      if (!((written >> r) & 1ull)) ws.clear(out + (long)r * ws.n1 * W);
+  }
+};
+
+// Value and gradient of one polynomial of a system by one warp into out.
+// A row's coefficients may be updated by different lanes in different
+// monomials; a row is touched at most once per monomial, and a warp barrier
+// ends each.
+template <class N, bool BIG>
+__device__ __forceinline__ void warp_poly_evaldiff(int dim, int deg, int maxvar, int m0, int m1,
+                                                   const int *__restrict__ nvr, const int *__restrict__ idx,
+                                                   const int *__restrict__ exps, const double *__restrict__ cst,
+                                                   const double *__restrict__ cff, const double *X, double *scr,
+                                                   double *out) {
+  const wser<N, BIG> ws(deg, threadIdx.x & 31);
+  const long S = (long)ws.n1 * N::width;
+  row_sink<N, BIG> sink(ws, out, scr + warp_slots(maxvar) * S, dim, cst);
+  for (int mon = m0; mon < m1; ++mon)
+    warp_monomial<N, BIG>(ws, dim, maxvar, nvr[mon], idx + (long)mon * maxvar, exps + (long)mon * maxvar,
+                          cff + mon * S, X, scr, sink);
+  sink.finish(dim);
+}
+
+// Sink of a warp that does one of a polynomial's monomials: the value and
+// the derivatives, scaled, in the warp's own series (slot 0 the value, slot
+// 1 + v the derivative in the monomial's variable v).
+template <class N, bool BIG>
+struct slot_sink {
+  typedef typename N::T T;
+  static const int W = N::width;
+  const wser<N, BIG> &ws;
+  double *slots;
+  __device__ __forceinline__ slot_sink(const wser<N, BIG> &w, double *s) : ws(w), slots(s) {}
+  __device__ __forceinline__ void value(int k, const T &z) { md::stn(slots + k * W, z); }
+  __device__ __forceinline__ void open(int) {}
+  __device__ __forceinline__ void derivative(int v, int, int e, int k, const T &z) {
+    md::stn(slots + ((1 + v) * ws.n1 + k) * W, (e > 1) ? N::scale_d(z, (double)e) : z);
+  }
+};
+
+// Value and gradient of one polynomial by all warps of a CTA, a monomial per
+// warp and round.  After each round the threads add the round's values and
+// derivatives to the rows (dim+1 series of shared memory) in the order of
+// the monomials, a thread per coefficient of every ng-th row, so a result
+// does not depend on the warps' timing.  scr: per warp warp_slots(maxvar)
+// scratch series and maxvar + 1 result series.
+template <class N, bool BIG>
+__device__ __forceinline__ void cta_poly_evaldiff(int dim, int deg, int maxvar, int m0, int m1,
+                                                  const int *__restrict__ nvr, const int *__restrict__ idx,
+                                                  const int *__restrict__ exps, const double *__restrict__ cst,
+                                                  const double *__restrict__ cff, const double *X, double *scr,
+                                                  double *rows, double *out) {
+  typedef typename N::T T;
+  const int W = N::width;
+  const wser<N, BIG> ws(deg, threadIdx.x & 31);
+  const int S = ws.n1 * W;
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int per = warp_slots(maxvar) + maxvar + 1;  // series per warp
+  double *mine = scr + (long)warp * per * S;
+  __shared__ int kdone[32];
+  for (int t = threadIdx.x; t < (dim + 1) * S; t += blockDim.x) rows[t] = t < dim * S ? 0.0 : cst[t - dim * S];
+  // thread t adds coefficient t mod n1 (and + blockDim when a series is
+  // longer than the CTA) of the rows g, g + ng, ...
+  const int ng = (int)blockDim.x / ws.n1 > 0 ? (int)blockDim.x / ws.n1 : 1;
+  const int g = (int)threadIdx.x / ws.n1;
+  for (int b = m0; b < m1; b += nw) {
+    const int mon = b + warp;
+    int k = 0;
+    if (mon < m1) {
+      slot_sink<N, BIG> sink(ws, mine + warp_slots(maxvar) * S);
+      k = warp_monomial<N, BIG>(ws, dim, maxvar, nvr[mon], idx + (long)mon * maxvar, exps + (long)mon * maxvar,
+                                cff + (long)mon * S, X, mine, sink);
+    }
+    if ((threadIdx.x & 31) == 0) kdone[warp] = k;
+    __syncthreads();
+    if (g < ng) {
+      for (int c = (int)threadIdx.x - g * ws.n1; c < ws.n1; c += blockDim.x) {
+        for (int w = 0; w < nw; ++w) {
+          const int kw = kdone[w];
+          const int *ix = idx + (long)(b + w) * maxvar;
+          const double *res = scr + ((long)w * per + warp_slots(maxvar)) * S + c * W;
+          for (int v = 0; v <= kw && kw > 0; ++v) {
+            const int r = v == 0 ? dim : ix[v - 1];
+            if (r % ng != g) continue;
+            T o, z;
+            double *row = rows + (long)r * S + c * W;
+            md::ldn(row, o);
+            md::ldn(res + (long)v * S, z);
+            md::stn(row, N::add(o, z));
+          }
+        }
       }
     }
-    __syncwarp();
+    __syncthreads();
   }
-  for (int k = lane; k < n1; k += 32) {
-    T v;
-    md::ldn(Vs + k * W, v);
-    md::stn(out + dim * S + k * W, v);
-  }
-  for (int r = 0; r < dim && r < 64; ++r)
-    if (!((written >> r) & 1ull))
-      for (int k = lane; k < n1; k += 32) md::stn(out + r * S + k * W, N::zero());
+  for (int t = threadIdx.x; t < (dim + 1) * S; t += blockDim.x) out[t] = rows[t];
 }
 
 }  // namespace phc
