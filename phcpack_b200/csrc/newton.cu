@@ -6,7 +6,8 @@
 // Newton/dbl2_newton_method.cpp:429 (dbl2_row_newton_qrstep) and :134
 // (dbl2_update_newton_qrstep), Newton/dbl2_systems_host.cpp:709
 // (dbl2_map_evaldiff_output), Newton/dbl2_newton_testers.cpp:116
-// (dbl2_update_series).  Four launches, all device-resident and capturable
+// (dbl2_update_series).  Four launches (and three more to pack the series when
+// the working degree is below the storage's), all device-resident and capturable
 // in one CUDA graph; the reference copies every intermediate to the host.
 #include "common.cuh"
 #include "dense.cuh"
@@ -32,9 +33,10 @@ __global__ void k_pack_series(long nseries, int W, int deg, int maxdeg, const do
   }
 }
 
-// output[s][i][j][k] (j = dim: value) -> jac[s][k][i][j], rhs[s][k][i] = -value
+// output[s][i][j][k] (j = dim: value) -> jac[s][k][i][j], rhs[s][k][i] = -value;
+// sol[s][k][i] = 0 (the least-squares solve leaves skipped blocks alone)
 __global__ void k_linearize(int nsys, int dim, int deg, int W, const double *__restrict__ out,
-                            double *__restrict__ jac, double *__restrict__ rhs) {
+                            double *__restrict__ jac, double *__restrict__ rhs, double *__restrict__ sol) {
   const int n1 = deg + 1;
   const long per = (long)dim * (dim + 1) * n1;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < (long)nsys * per; t += (long)gridDim.x * blockDim.x) {
@@ -48,8 +50,11 @@ __global__ void k_linearize(int nsys, int dim, int deg, int W, const double *__r
       double *dst = jac + ((((s * n1 + k) * dim + i) * dim) + j) * W;
       for (int c = 0; c < W; ++c) dst[c] = src[c];
     } else {
-      double *dst = rhs + ((s * n1 + k) * dim + i) * W;
-      for (int c = 0; c < W; ++c) dst[c] = -src[c];
+      const long o = ((s * n1 + k) * dim + i) * W;
+      for (int c = 0; c < W; ++c) {
+        rhs[o + c] = -src[c];
+        sol[o + c] = 0.0;
+      }
     }
   }
 }
@@ -110,16 +115,23 @@ int newton_step(int prec, int cplx, int nsys, int dim, int deg, int maxdeg, int 
   double *sol = p;  p += (long)nsys * n1 * dim * W;
   double *bw = p;
   const int T = 256;
-  k_pack_series<<<grid_for((long)nsys * dim * n1 * W, T), T, 0, st>>>((long)nsys * dim, (int)W, deg, maxdeg, series, xin);
-  k_pack_series<<<grid_for((long)nsys * dim * n1 * W, T), T, 0, st>>>((long)nsys * dim, (int)W, deg, maxdeg, cst, cs);
-  if (nmon > 0)
-    k_pack_series<<<grid_for(nmon * n1 * W, T), T, 0, st>>>(nmon, (int)W, deg, maxdeg, cff, cf);
-  PHC_CHECK_LAUNCH();
-  int rc = system_evaldiff(prec, cplx, nsys, dim, deg, maxvar, mon_off, nvr, idx, exps, cs, cf, xin, out, st);
+  // at the full degree the series are contiguous already: no packing (three
+  // launches of the seven of a step on one small system)
+  const double *ecst = cst, *ecff = cff, *ein = series;
+  if (deg < maxdeg) {
+    k_pack_series<<<grid_for((long)nsys * dim * n1 * W, T), T, 0, st>>>((long)nsys * dim, (int)W, deg, maxdeg, series, xin);
+    k_pack_series<<<grid_for((long)nsys * dim * n1 * W, T), T, 0, st>>>((long)nsys * dim, (int)W, deg, maxdeg, cst, cs);
+    if (nmon > 0)
+      k_pack_series<<<grid_for(nmon * n1 * W, T), T, 0, st>>>(nmon, (int)W, deg, maxdeg, cff, cf);
+    PHC_CHECK_LAUNCH();
+    ecst = cs;
+    ecff = cf;
+    ein = xin;
+  }
+  int rc = system_evaldiff(prec, cplx, nsys, dim, deg, maxvar, mon_off, nvr, idx, exps, ecst, ecff, ein, out, st);
   if (rc) return rc;
-  k_linearize<<<grid_for((long)nsys * dim * (dim + 1) * n1, T), T, 0, st>>>(nsys, dim, deg, (int)W, out, jac, rhs);
+  k_linearize<<<grid_for((long)nsys * dim * (dim + 1) * n1, T), T, 0, st>>>(nsys, dim, deg, (int)W, out, jac, rhs, sol);
   PHC_CHECK_LAUNCH();
-  PHC_CUDA(cudaMemsetAsync(sol, 0, (size_t)nsys * n1 * dim * W * sizeof(double), st));
   rc = bals_solve(prec, cplx, nsys, dim, (int)n1, szt, -1, jac, rhs, sol, Q, R, flags, bw, st);
   if (rc) return rc;
 #define PHC_UPD(R_, C_)                                                                                         \
