@@ -15,7 +15,7 @@ __host__ __device__ inline long dense_stride(int n, int szt, int W, bool oz) {
 }
 
 template <class N, bool OZ>
-__global__ void __launch_bounds__(kDenseThreads)
+__global__ void __launch_bounds__(kDenseThreads, 2)
     k_blocked_houseqr(int n, int ncols, int szt, const double *__restrict__ A, double *__restrict__ Q,
                       double *__restrict__ Rm, double *__restrict__ work, int stage) {
   extern __shared__ __align__(16) double sm[];
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kDenseThreads)
 // overwritten by the updated right hand sides and the diagonal tiles of U by
 // their inverses.
 template <class N>
-__global__ void __launch_bounds__(kDenseThreads)
+__global__ void __launch_bounds__(kDenseThreads, 2)
     k_upper_tiled_solver(int dim, int szt, double *__restrict__ U, double *__restrict__ b, double *__restrict__ x,
                          double *__restrict__ work) {
   const int W = N::width;
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kDenseThreads)
 // flags per instance: zeroQ, noqr, upidx, bsidx, newtail; with tailidx < 0
 // the tail starts at the instance's flags[4].
 template <class N, bool OZ>
-__global__ void __launch_bounds__(kDenseThreads)
+__global__ void __launch_bounds__(kDenseThreads, 2)
     k_bals_solve(int n, int degp1, int szt, int tailidx, const double *__restrict__ mat, double *__restrict__ rhs,
                  double *__restrict__ sol, double *__restrict__ Q, double *__restrict__ Rm, int *__restrict__ flags,
                  double *__restrict__ work, int stage) {
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kDenseThreads)
   const int tail0 = max(1, tailidx >= 0 ? tailidx : fl[4]);
   bool tinv_ok = false;
   if (!(noqr && !zeroQ)) {
-    const double nrm = block_maxnorm<N>(n, b, S.red);
+    const double nrm = warp_maxnorm<N>(n, b);
     if (head_tiny<N>(nrm)) {
       noqr = zeroQ ? 0 : 1;
       if (noqr)
@@ -115,22 +115,27 @@ __global__ void __launch_bounds__(kDenseThreads)
     if (!tinv_ok) block_invert_tiles<N>(n, szt, r, n, tinv);
     bool first = true;
     newtail = degp1;
+    // S.x holds x_{i-1} at the start of stage i
+    __syncthreads();
+    for (int l = threadIdx.x; l < n; l += blockDim.x)
+      stn_at<N>(S.x, l, ldn_at<N>(x, (long)(tail0 - 1) * n + l));
+    __syncthreads();
     for (int i = tail0; i < degp1; ++i) {
-      const double *xp = x + (long)(i - 1) * n * W;
-      double nrm = block_maxnorm<N>(n, xp, S.red);
-      if (nrm < skip_tol<N>()) {
+      double nrm = warp_maxnorm<N>(n, S.x);
+      if (nrm < skip_tol<N>())
         ++up;
-      } else {
-        for (int l = threadIdx.x; l < n; l += blockDim.x) stn_at<N>(S.x, l, ldn_at<N>(xp, l));
-        __syncthreads();
+      else
         block_tail_update<N>(n, degp1, i, A, b, S.x);
-      }
       const double *bi = b + (long)i * n * W;
-      nrm = block_maxnorm<N>(n, bi, S.red);
+      nrm = warp_maxnorm<N>(n, bi);
       double *xi = x + (long)i * n * W;
       if (nrm < skip_tol<N>()) {
         ++bs;
-        for (int l = threadIdx.x; l < n; l += blockDim.x) stn_at<N>(xi, l, N::zero());
+        __syncthreads();  // every warp has read S.x
+        for (int l = threadIdx.x; l < n; l += blockDim.x) {
+          stn_at<N>(S.x, l, N::zero());
+          stn_at<N>(xi, l, N::zero());
+        }
         __syncthreads();
       } else {
         if (first) {
@@ -140,7 +145,6 @@ __global__ void __launch_bounds__(kDenseThreads)
         block_qhb<N>(n, q, bi, S.w);
         block_tiled_backsub<N>(n, szt, r, n, tinv, S.w, S.x);
         for (int l = threadIdx.x; l < n; l += blockDim.x) stn_at<N>(xi, l, ldn_at<N>(S.x, l));
-        __syncthreads();
       }
     }
   }
@@ -201,7 +205,7 @@ __device__ __forceinline__ void residue_dec(typename N::T &r, const typename N::
 }
 
 template <class N>
-__global__ void __launch_bounds__(kDenseThreads)
+__global__ void __launch_bounds__(kDenseThreads, 2)
     k_linear_residue(int n, int degp1, int tailidx, const double *__restrict__ mat, const double *__restrict__ rhs,
                      const double *__restrict__ sol, double *__restrict__ res, double *__restrict__ resmax) {
   typedef typename N::T T;

@@ -81,12 +81,15 @@ __device__ __forceinline__ double block_min(double a, double *red) {
 }
 
 // max_i |leading limb| of v (complex: |re| + |im|): the "1-norm" of the
-// reference's skip rules, Newton/dbl_onenorms_host.cpp:9,20
+// reference's skip rules, Newton/dbl_onenorms_host.cpp:9,20.  Every warp
+// forms it by itself (n is at most a few dozen: a CTA-wide reduction would
+// cost three barriers for two loads per lane), so all threads get the result
+// without a barrier.
 template <class N>
-__device__ double block_maxnorm(int n, const double *v, double *red) {
+__device__ __forceinline__ double warp_maxnorm(int n, const double *v) {
   double a = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) a = fmax(a, N::lead(ldn_at<N>(v, i)));
-  return block_max(a, red);
+  for (int i = threadIdx.x & 31; i < n; i += 32) a = fmax(a, N::lead(ldn_at<N>(v, i)));
+  return warp_max(a);
 }
 
 // Skip thresholds of the reference's least-squares solvers per precision:
@@ -146,26 +149,66 @@ __device__ __forceinline__ typename N::T group4_sum(typename N::T a) {
   return N::add(a, md::shfl_xor(a, 2));
 }
 
-// ------------------------------------------------------------- Householder
-// Reflector of x = R[c.., c], m = n - c entries, in PHCpack's convention
-// (Matrices/dbl2_factorizations.cpp:374 real, :436 complex): v[0] = 1,
-// beta = 2|v0|^2/(sigma + |v0|^2); the real case takes v0 = x0 - mu or
-// -sigma/(x0 + mu), the complex case v0 = x0 - mu x0/|x0|.
-// Leaves v in S.v (m numbers) and beta in S.misc[0] (real part of a number).
+// The same with groups of 8 lanes, for long chains.
 template <class N>
-__device__ void block_house(int m, const double *col, long ld, dense_smem &S) {
+__device__ __forceinline__ typename N::T group_sum(typename N::T a, int lanes) {
+  a = group4_sum<N>(a);
+  return lanes == 8 ? N::add(a, md::shfl_xor(a, 4)) : a;
+}
+
+// ------------------------------------------------------------- Householder
+// One column of a panel: the reflector of x = R[c.., c], m = n - c entries,
+// in PHCpack's convention (Matrices/dbl2_factorizations.cpp:374 real, :436
+// complex): v[0] = 1, beta = 2|v0|^2/(sigma + |v0|^2); the real case takes
+// v0 = x0 - mu or -sigma/(x0 + mu), the complex case v0 = x0 - mu x0/|x0|;
+// and R[c.., c..e) <- (I - beta v v^H) R[c.., c..e), w_j = beta sum_i
+// conj(R_ij) v_i, R_ij -= v_i conj(w_j) (:534/:567).
+//
+// A reflector is a chain of dependent scalar operations (a square root and
+// two divisions, most of a quad-double column's time) between two sweeps
+// over the panel.  With v = (1, x_i / v0) the inner products split into
+// conj(R_cj) + (1/v0) D_j, D_j = sum_{i>c} conj(R_ij) x_i, and D_c is sigma
+// itself: the first sweep needs nothing of the chain and also replaces the
+// norm's reduction, and the warps 0 and 1 form beta and 1/v0 side by side.
+// Four barriers per column.  Entry (i, j) of R sits at Rm[(i - r0) * ld +
+// (j - c0)]: the whole matrix (r0 = c0 = 0, ld = ncols) or a panel of it
+// staged in shared memory.  Leaves v in S.v (m numbers) and beta in
+// S.misc[0] (a real number).
+template <class N>
+__device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_smem &S, int r0, int c0) {
   typedef typename N::T T;
   typedef typename N::real R;
   typedef md::num<R, false> RN;
-  R sig = RN::zero();
-  for (int i = 1 + threadIdx.x; i < m; i += blockDim.x) {
-    const T xi = ldn_at<N>(col, (long)i * ld);
-    sig = RN::add(sig, N::norm2(xi));
-    stn_at<N>(S.v, i, xi);
+  const int m = n - c, nc = e - c;
+  double *col = Rm + ((long)(c - r0) * ld + (c - c0)) * N::width;  // entry (c, c)
+  {
+    // D_j for the panel's columns, 4 lanes per column (8 when the columns
+    // are few and long)
+    const int G = (nc * 8 <= (int)blockDim.x && m > 16) ? 8 : 4;
+    const int grp = threadIdx.x / G, part = threadIdx.x % G, ngrp = blockDim.x / G;
+    for (int base = 0; base < nc; base += ngrp) {
+      const int j = base + grp;
+      md::msum<N> sum;
+      sum.zero();
+      if (j < nc)
+        for (int i = 1 + part; i < m; i += G) sum.cfma(ldn_at<N>(col, (long)i * ld + j), ldn_at<N>(col, (long)i * ld));
+      const T d = group_sum<N>(sum.value(), G);
+      if (j < nc && part == 0) stn_at<N>(S.w, j, d);
+    }
   }
-  const R sigma = block_sum<RN>(sig, S.red);
-  if (threadIdx.x == 0) {
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  if (warp < 2) {
     const T x0 = ldn_at<N>(col, 0);
+    R sigma;
+    {
+      const T d0 = ldn_at<N>(S.w, 0);
+      if constexpr (N::is_complex)
+        sigma = d0.re;
+      else
+        sigma = d0;
+    }
+    const bool do_beta = warp == 0, do_inv = warp == 1 || nwarp == 1;
     R beta = RN::zero();
     T inv = N::one();
     if (!md::is_zero(sigma)) {
@@ -182,66 +225,54 @@ __device__ void block_house(int m, const double *col, long ld, dense_smem &S) {
         }
       } else {
         const R mu = RN::tr::sqrt(RN::add(RN::mul(x0, x0), sigma));
-        if (md::lead(x0) <= 0.0)
-          v0 = RN::sub(x0, mu);
-        else
-          v0 = RN::neg(RN::tr::div(sigma, RN::add(x0, mu)));
+        const bool cancel = !(md::lead(x0) <= 0.0);  // x0 - mu would cancel
+        const R a = cancel ? RN::add(x0, mu) : RN::sub(x0, mu);
+        if (cancel) {
+          if (do_inv) inv = RN::neg(RN::tr::div(a, sigma));
+          v0 = do_beta ? RN::neg(RN::tr::div(sigma, a)) : a;
+        } else {
+          if (do_inv) inv = RN::tr::div(RN::one(), a);
+          v0 = a;
+        }
       }
       const R v0sq = N::norm2(v0);
-      beta = md::mul_d(RN::tr::div(v0sq, RN::add(sigma, v0sq)), 2.0);
+      if (do_beta) beta = md::mul_d(RN::tr::div(v0sq, RN::add(sigma, v0sq)), 2.0);
       if constexpr (N::is_complex) {
-        inv = N::mkc(RN::tr::div(v0.re, v0sq), RN::neg(RN::tr::div(v0.im, v0sq)));
-      } else {
-        inv = v0;  // the real case divides by v0
+        if (do_inv) inv = N::mkc(RN::tr::div(v0.re, v0sq), RN::neg(RN::tr::div(v0.im, v0sq)));
       }
     }
-    stn_at<RN>(S.misc, 0, beta);
-    stn_at<N>(S.misc + 2 * N::width, 0, inv);
-  }
-  __syncthreads();
-  const R beta = ldn_at<RN>(S.misc, 0);
-  const T inv = ldn_at<N>(S.misc + 2 * N::width, 0);
-  if (!md::is_zero(beta)) {
-    for (int i = 1 + threadIdx.x; i < m; i += blockDim.x) {
-      const T vi = ldn_at<N>(S.v, i);
-      if constexpr (N::is_complex)
-        stn_at<N>(S.v, i, N::mul(vi, inv));
-      else
-        stn_at<N>(S.v, i, N::div(vi, inv));
+    if ((threadIdx.x & 31) == 0) {
+      if (do_beta) stn_at<RN>(S.misc, 0, beta);
+      if (do_inv) stn_at<N>(S.misc + 2 * N::width, 0, inv);
     }
   }
-  if (threadIdx.x == 0) stn_at<N>(S.v, 0, N::one());
   __syncthreads();
-}
-
-// R[c.., c..e) <- (I - beta v v^H) R[c.., c..e): w_j = beta sum_i conj(R_ij) v_i,
-// R_ij -= v_i conj(w_j)   (Matrices/dbl2_factorizations.cpp:534/:567).
-// Entry (i, j) of R sits at Rm[(i - r0) * ld + (j - c0)]: the whole matrix
-// (r0 = c0 = 0, ld = ncols) or a panel of it staged in shared memory.
-template <class N>
-__device__ void block_apply_reflector(int n, long ld, int c, int e, double *Rm, dense_smem &S, int r0 = 0,
-                                      int c0 = 0) {
-  typedef typename N::T T;
-  typedef typename N::real R;
-  typedef md::num<R, false> RN;
-  const int grp = threadIdx.x >> 2, part = threadIdx.x & 3, ngrp = blockDim.x >> 2;
   const R beta = ldn_at<RN>(S.misc, 0);
-  if (md::is_zero(beta)) return;
-  for (int base = c; base < e; base += ngrp) {  // four lanes per column
-    const int j = base + grp;
-    T acc = N::zero();
-    if (j < e)
-      for (int i = c + part; i < n; i += 4)
-        acc = N::add(acc, N::mul(N::conj(ldn_at<N>(Rm, (long)(i - r0) * ld + (j - c0))), ldn_at<N>(S.v, i - c)));
-    acc = group4_sum<N>(acc);
-    if (j < e && part == 0) stn_at<N>(S.w, j - c, N::scale(acc, beta));
+  const bool trivial = md::is_zero(beta);
+  // v (as the reference leaves it when there is nothing to reflect) and w
+  {
+    const T inv = ldn_at<N>(S.misc + 2 * N::width, 0);
+    for (int t = threadIdx.x; t < m + nc; t += blockDim.x) {
+      if (t < m) {
+        T v = N::one();
+        if (t > 0) {
+          v = ldn_at<N>(col, (long)t * ld);
+          if (!trivial) v = N::mul(v, inv);
+        }
+        stn_at<N>(S.v, t, v);
+      } else if (!trivial) {
+        const int j = t - m;
+        const T d = md::mul_add<N>(N::conj(ldn_at<N>(col, j)), inv, ldn_at<N>(S.w, j));
+        stn_at<N>(S.w, j, N::scale(d, beta));
+      }
+    }
   }
   __syncthreads();
-  const int nc = e - c;
-  for (int t = threadIdx.x; t < (n - c) * nc; t += blockDim.x) {
-    const int i = c + t / nc, j = c + t % nc;
-    const long o = (long)(i - r0) * ld + (j - c0);
-    stn_at<N>(Rm, o, N::sub(ldn_at<N>(Rm, o), N::mul(ldn_at<N>(S.v, i - c), N::conj(ldn_at<N>(S.w, j - c)))));
+  if (trivial) return;
+  for (int t = threadIdx.x; t < m * nc; t += blockDim.x) {
+    const int i = t / nc, j = t - i * nc;
+    const long o = (long)i * ld + j;
+    stn_at<N>(col, o, md::mul_sub<N>(ldn_at<N>(col, o), ldn_at<N>(S.v, i), N::conj(ldn_at<N>(S.w, j))));
   }
   __syncthreads();
 }
@@ -288,13 +319,10 @@ __device__ void block_houseqr(int n, int ncols, int szt, double *Q, double *Rm, 
     }
     for (int L = 0; L < szt; ++L) {
       const int c = rowoff + L;
-      if (panel) {
-        block_house<N>(n - c, panel + ((long)L * szt + L) * W, szt, S);
-        block_apply_reflector<N>(n, szt, c, endcol, panel, S, rowoff, rowoff);
-      } else {
-        block_house<N>(n - c, Rm + (long)c * ncols * W + (long)c * W, ncols, S);
-        block_apply_reflector<N>(n, ncols, c, endcol, Rm, S);
-      }
+      if (panel)
+        block_reflect<N>(n, szt, c, endcol, panel, S, rowoff, rowoff);
+      else
+        block_reflect<N>(n, ncols, c, endcol, Rm, S, 0, 0);
       if (threadIdx.x == 0) stn_at<RN>(S.beta, L, ldn_at<RN>(S.misc, 0));
       for (int i = threadIdx.x; i < m; i += blockDim.x)
         stn_at<N>(Y, (long)L * m + i, (i < L) ? N::zero() : ldn_at<N>(S.v, i - L));
@@ -305,30 +333,44 @@ __device__ void block_houseqr(int n, int ncols, int szt, double *Q, double *Rm, 
         stn_at<N>(Rm, (long)(rowoff + t / szt) * ncols + rowoff + t % szt, ldn_at<N>(panel, t));
       __syncthreads();
     }
-    // W from the betas and Y (Matrices/dbl2_baqr_host.cpp:13)
+    // W from the betas and Y (Matrices/dbl2_baqr_host.cpp:13): w_j = -beta_j
+    // (y_j + sum_{l<j} w_l (y_l^H y_j)).  The inner products y_l^H y_j do not
+    // wait for the w: all of them first (in P and T, free until the trailing
+    // products; szt^2 <= 2 n szt numbers), then the columns one after another
+    // with 4 lanes per entry.  y_l starts at row l.
     {
+      const int grp = threadIdx.x >> 2, part = threadIdx.x & 3, ngrp = blockDim.x >> 2;
+      const int pairs = szt * (szt - 1) / 2;
+      int j = 1, kk = grp;  // pair number grp: (kk, j), kk < j
+      while (j < szt && kk >= j) kk -= j++;
+      for (int base = 0; base < pairs; base += ngrp) {
+        const bool on = base + grp < pairs;
+        md::msum<N> sum;
+        sum.zero();
+        if (on)
+          for (int i = j + part; i < m; i += 4)
+            sum.cfma(ldn_at<N>(Y, (long)kk * m + i), ldn_at<N>(Y, (long)j * m + i));
+        const T g = group4_sum<N>(sum.value());
+        if (on && part == 0) stn_at<N>(P, (long)j * szt + kk, g);
+        kk += ngrp;
+        while (j < szt && kk >= j) kk -= j++;
+      }
       const R b0 = ldn_at<RN>(S.beta, 0);
       for (int i = threadIdx.x; i < m; i += blockDim.x)
         stn_at<N>(Wm, i, N::neg(N::scale(ldn_at<N>(Y, i), b0)));
       __syncthreads();
-      const int grp = threadIdx.x >> 2, part = threadIdx.x & 3, ngrp = blockDim.x >> 2;
-      for (int j = 1; j < szt; ++j) {
-        for (int base = 0; base < j; base += ngrp) {  // four lanes per inner product
-          const int kk = base + grp;
-          T acc = N::zero();
-          if (kk < j)
-            for (int i = part; i < m; i += 4)
-              acc = N::add(acc, N::mul(N::conj(ldn_at<N>(Y, (long)kk * m + i)), ldn_at<N>(Y, (long)j * m + i)));
-          acc = group4_sum<N>(acc);
-          if (kk < j && part == 0) stn_at<N>(S.w, kk, acc);
-        }
-        __syncthreads();
-        const R bj = ldn_at<RN>(S.beta, j);
-        for (int i = threadIdx.x; i < m; i += blockDim.x) {
-          T z = N::zero();
-          for (int kk = 0; kk < j; ++kk) z = N::add(z, N::mul(ldn_at<N>(Wm, (long)kk * m + i), ldn_at<N>(S.w, kk)));
-          z = N::add(z, ldn_at<N>(Y, (long)j * m + i));
-          stn_at<N>(Wm, (long)j * m + i, N::neg(N::scale(z, bj)));
+      for (int jj = 1; jj < szt; ++jj) {
+        const R bj = ldn_at<RN>(S.beta, jj);
+        for (int base = 0; base < m; base += ngrp) {
+          const int i = base + grp;
+          md::msum<N> z;
+          z.zero();
+          if (i < m) {
+            if (part == 0) z.set(ldn_at<N>(Y, (long)jj * m + i));
+            for (int l = part; l < jj; l += 4) z.fma(ldn_at<N>(Wm, (long)l * m + i), ldn_at<N>(P, (long)jj * szt + l));
+          }
+          const T zz = group4_sum<N>(z.value());
+          if (i < m && part == 0) stn_at<N>(Wm, (long)jj * m + i, N::neg(N::scale(zz, bj)));
         }
         __syncthreads();
       }
@@ -364,39 +406,43 @@ __device__ void block_houseqr(int n, int ncols, int szt, double *Q, double *Rm, 
       const int nc = ncols - endcol;
       for (int t = threadIdx.x; t < szt * nc; t += blockDim.x) {
         const int kk = t / nc, j = t % nc;
-        T acc = N::zero();
+        md::msum<N> acc;
+        acc.zero();
         for (int i = 0; i < m; ++i)
-          acc = N::add(acc, N::mul(N::conj(ldn_at<N>(Wm, (long)kk * m + i)),
-                                   ldn_at<N>(Rm, (long)(rowoff + i) * ncols + endcol + j)));
-        stn_at<N>(P, (long)kk * nc + j, acc);
+          acc.cfma(ldn_at<N>(Wm, (long)kk * m + i), ldn_at<N>(Rm, (long)(rowoff + i) * ncols + endcol + j));
+        stn_at<N>(P, (long)kk * nc + j, acc.value());
       }
       __syncthreads();
       for (int t = threadIdx.x; t < m * nc; t += blockDim.x) {
         const int i = t / nc, j = t % nc;
-        T acc = N::zero();
-        for (int kk = 0; kk < szt; ++kk)
-          acc = N::add(acc, N::mul(ldn_at<N>(Y, (long)kk * m + i), ldn_at<N>(P, (long)kk * nc + j)));
         const long o = (long)(rowoff + i) * ncols + endcol + j;
-        stn_at<N>(Rm, o, N::add(ldn_at<N>(Rm, o), acc));
+        md::msum<N> acc;
+        acc.set(ldn_at<N>(Rm, o));
+        for (int kk = 0; kk < szt; ++kk) acc.fma(ldn_at<N>(Y, (long)kk * m + i), ldn_at<N>(P, (long)kk * nc + j));
+        stn_at<N>(Rm, o, acc.value());
       }
       __syncthreads();
     }
     // Q[:, rowoff..] += (Q[:, rowoff..] W) Y^H
     for (int t = threadIdx.x; t < n * szt; t += blockDim.x) {
       const int i = t / szt, kk = t % szt;
-      T acc = N::zero();
-      for (int l = 0; l < m; ++l)
-        acc = N::add(acc, N::mul(ldn_at<N>(Q, (long)i * n + rowoff + l), ldn_at<N>(Wm, (long)kk * m + l)));
-      stn_at<N>(Tm, (long)i * szt + kk, acc);
+      if (k == 0) {  // Q is still the identity
+        stn_at<N>(Tm, (long)i * szt + kk, ldn_at<N>(Wm, (long)kk * m + i));
+        continue;
+      }
+      md::msum<N> acc;
+      acc.zero();
+      for (int l = 0; l < m; ++l) acc.fma(ldn_at<N>(Q, (long)i * n + rowoff + l), ldn_at<N>(Wm, (long)kk * m + l));
+      stn_at<N>(Tm, (long)i * szt + kk, acc.value());
     }
     __syncthreads();
     for (int t = threadIdx.x; t < n * m; t += blockDim.x) {
       const int i = t / m, j = t % m;
-      T acc = N::zero();
-      for (int kk = 0; kk < szt; ++kk)
-        acc = N::add(acc, N::mul(ldn_at<N>(Tm, (long)i * szt + kk), N::conj(ldn_at<N>(Y, (long)kk * m + j))));
       const long o = (long)i * n + rowoff + j;
-      stn_at<N>(Q, o, N::add(ldn_at<N>(Q, o), acc));
+      md::msum<N> acc;
+      acc.set(ldn_at<N>(Q, o));
+      for (int kk = 0; kk < szt; ++kk) acc.cfma(ldn_at<N>(Y, (long)kk * m + j), ldn_at<N>(Tm, (long)i * szt + kk));
+      stn_at<N>(Q, o, acc.value());
     }
     __syncthreads();
   }
@@ -404,24 +450,43 @@ __device__ void block_houseqr(int n, int ncols, int szt, double *Q, double *Rm, 
 
 // ------------------------------------------------------ tiled back substitution
 // Inverse of every szt x szt diagonal tile of the upper triangular U (dim x dim,
-// leading dimension ldu) into Tinv (nbt tiles of szt x szt), one thread per
+// leading dimension ldu) into Tinv (nbt tiles of szt x szt), four lanes per
 // (tile, column): column j of the inverse solves T x = e_j by back
 // substitution (Matrices/dbl2_tabs_host.cpp:31 CPU_dbl2_upper_inverse,
-// dbl2_tabs_kernels.cu:397 dbl2_invert_tiles).
+// dbl2_tabs_kernels.cu:397 dbl2_invert_tiles).  A column is a chain of szt
+// rows; the rows' reciprocal pivots, a division each, are formed beforehand
+// side by side (kept on the diagonal of Tinv until the row is reached by its
+// own column, whose entry they are).
 template <class N>
 __device__ void block_invert_tiles(int dim, int szt, const double *U, int ldu, double *Tinv) {
   typedef typename N::T T;
-  const int nbt = dim / szt;
-  for (int t = threadIdx.x; t < nbt * szt; t += blockDim.x) {
-    const int tile = t / szt, j = t % szt;
+  const int W = N::width;
+  const long tile2 = (long)szt * szt;
+  for (int t = threadIdx.x; t < dim; t += blockDim.x) {
+    const int tile = t / szt, i = t - tile * szt;
+    stn_at<N>(Tinv, tile * tile2 + (long)i * szt + i, N::div(N::one(), ldn_at<N>(U, (long)t * ldu + t)));
+  }
+  __syncthreads();
+  const int grp = threadIdx.x >> 2, part = threadIdx.x & 3, ngrp = blockDim.x >> 2;
+  for (int base = 0; base < dim; base += ngrp) {
+    const int t = base + grp;
+    const int tile = t / szt, j = t < dim ? t - tile * szt : 0;
     const int off = tile * szt;
-    double *inv = Tinv + (long)tile * szt * szt * N::width;
-    for (int i = szt - 1; i > j; --i) stn_at<N>(inv, (long)i * szt + j, N::zero());
-    for (int i = j; i >= 0; --i) {
-      T acc = (i == j) ? N::one() : N::zero();
-      for (int l = j; l > i; --l)
-        acc = N::sub(acc, N::mul(ldn_at<N>(U, (long)(off + i) * ldu + off + l), ldn_at<N>(inv, (long)l * szt + j)));
-      stn_at<N>(inv, (long)i * szt + j, N::div(acc, ldn_at<N>(U, (long)(off + i) * ldu + off + i)));
+    double *inv = Tinv + tile * tile2 * W;
+    if (t < dim)
+      for (int i = j + 1 + part; i < szt; i += 4) stn_at<N>(inv, (long)i * szt + j, N::zero());
+    // rows above the diagonal entry, all groups of the warp in step
+    for (int back = 1; back < szt; ++back) {
+      const int i = j - back;
+      const bool on = t < dim && i >= 0;
+      md::msum<N> sum;
+      sum.zero();
+      if (on)
+        for (int l = j - part; l > i; l -= 4)
+          sum.fnma(ldn_at<N>(U, (long)(off + i) * ldu + off + l), ldn_at<N>(inv, (long)l * szt + j));
+      const T acc = group4_sum<N>(sum.value());
+      if (on && part == 0) stn_at<N>(inv, (long)i * szt + j, N::mul(acc, ldn_at<N>(inv, (long)i * szt + i)));
+      __syncwarp();
     }
   }
   __syncthreads();
@@ -441,21 +506,21 @@ __device__ void block_tiled_backsub(int dim, int szt, const double *U, int ldu, 
     const double *inv = Tinv + (long)k * szt * szt * N::width;
     for (int base = 0; base < szt; base += ngrp) {
       const int i = base + grp;
-      T acc = N::zero();
+      md::msum<N> sum;
+      sum.zero();
       if (i < szt)
-        for (int j = part; j < szt; j += 4)
-          acc = N::add(acc, N::mul(ldn_at<N>(inv, (long)i * szt + j), ldn_at<N>(b, off + j)));
-      acc = group4_sum<N>(acc);
+        for (int j = part; j < szt; j += 4) sum.fma(ldn_at<N>(inv, (long)i * szt + j), ldn_at<N>(b, off + j));
+      const T acc = group4_sum<N>(sum.value());
       if (i < szt && part == 0) stn_at<N>(x, off + i, acc);
     }
     __syncthreads();
     for (int base = 0; base < off; base += ngrp) {
       const int r = base + grp;
-      T acc = N::zero();
+      md::msum<N> sum;
+      sum.zero();
       if (r < off)
-        for (int j = part; j < szt; j += 4)
-          acc = N::add(acc, N::mul(ldn_at<N>(U, (long)r * ldu + off + j), ldn_at<N>(x, off + j)));
-      acc = group4_sum<N>(acc);
+        for (int j = part; j < szt; j += 4) sum.fma(ldn_at<N>(U, (long)r * ldu + off + j), ldn_at<N>(x, off + j));
+      const T acc = group4_sum<N>(sum.value());
       if (r < off && part == 0) stn_at<N>(b, r, N::sub(ldn_at<N>(b, r), acc));
     }
     __syncthreads();
@@ -470,42 +535,71 @@ __device__ void block_qhb(int n, const double *Q, const double *b, double *w) {
   const int grp = threadIdx.x >> 2, part = threadIdx.x & 3, ngrp = blockDim.x >> 2;
   for (int base = 0; base < n; base += ngrp) {
     const int i = base + grp;
-    T acc = N::zero();
+    md::msum<N> sum;
+    sum.zero();
     if (i < n)
-      for (int j = part; j < n; j += 4)
-        acc = N::add(acc, N::mul(N::conj(ldn_at<N>(Q, (long)j * n + i)), ldn_at<N>(b, j)));
-    acc = group4_sum<N>(acc);
+      for (int j = part; j < n; j += 4) sum.cfma(ldn_at<N>(Q, (long)j * n + i), ldn_at<N>(b, j));
+    const T acc = group4_sum<N>(sum.value());
     if (i < n && part == 0) stn_at<N>(w, i, acc);
   }
   __syncthreads();
 }
 
 // b_j -= A_{j-i+1} x for j = i..degp1-1 (Newton/dbl2_tail_kernels.cu:19
-// dbl2_bals_tail, all right hand sides of one stage at once): one thread per
-// row of the stacked matrices A_1 .. A_{degp1-i}, the row's dot product with
-// x (shared memory) in two interleaved partial sums.  The stage is a chain
-// of dependent multiple-double operations per row; a thread per row keeps
-// every thread of the CTA on its own chain instead of reducing each row
-// across a warp.
+// dbl2_bals_tail, all right hand sides of one stage at once), over the rows
+// of the stacked matrices A_1 .. A_{degp1-i}.  Quad-double: a thread per row
+// (its 450 FP64 cycles per product cover the uncoalesced loads), two or four
+// when the rows would leave threads idle.  Double and
+// double-double: four lanes per row, so that a load instruction touches 8
+// lines instead of 32 (a thread per row was bound by the L1 cache's
+// wavefronts) and a stage's rows fill the CTA.
 template <class N>
 __device__ void block_tail_update(int n, int degp1, int i, const double *mat, double *rhs, const double *x) {
   typedef typename N::T T;
   const long nn = (long)n * n;
   const int rows = (degp1 - i) * n;
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-    const int j = i + r / n, row = r % n;
-    const double *A = mat + (long)(j - i + 1) * nn * N::width + (long)row * n * N::width;
-    T a0 = N::zero(), a1 = N::zero();
-    int l = 0;
-    for (; l + 1 < n; l += 2) {
-      a0 = N::add(a0, N::mul(ldn_at<N>(A, l), ldn_at<N>(x, l)));
-      a1 = N::add(a1, N::mul(ldn_at<N>(A, l + 1), ldn_at<N>(x, l + 1)));
+  if constexpr (N::tr::limbs > 2) {
+    const int G = rows * 4 <= (int)blockDim.x ? 4 : (rows * 2 <= (int)blockDim.x ? 2 : 1);
+    const int grp = threadIdx.x / G, part = threadIdx.x % G, ngrp = blockDim.x / G;
+    for (int base = 0; base < rows; base += ngrp) {
+      const int r = base + grp;
+      const double *A = mat + (nn + (long)r * n) * N::width;
+      double *bj = rhs + ((long)i * n + r) * N::width;
+      md::msum<N> sum;
+      sum.zero();
+      if (r < rows) {
+        if (part == 0) {
+          T v;
+          md::ldn(bj, v);
+          sum.set(v);
+        }
+        for (int l = part; l < n; l += G) sum.fnma(ldn_at<N>(A, l), ldn_at<N>(x, l));
+      }
+      T v = sum.value();
+      if (G > 1) v = N::add(v, md::shfl_xor(v, 1));
+      if (G > 2) v = N::add(v, md::shfl_xor(v, 2));
+      if (r < rows && part == 0) md::stn(bj, v);
     }
-    if (l < n) a0 = N::add(a0, N::mul(ldn_at<N>(A, l), ldn_at<N>(x, l)));
-    double *bj = rhs + ((long)j * n + row) * N::width;
-    T v;
-    md::ldn(bj, v);
-    md::stn(bj, N::sub(v, N::add(a0, a1)));
+  } else {
+    const int grp = threadIdx.x >> 2, part = threadIdx.x & 3, ngrp = blockDim.x >> 2;
+    for (int base = 0; base < rows; base += ngrp) {
+      const int r = base + grp;
+      // the stacked matrices are contiguous: row r of A_1, A_2, ...
+      const double *A = mat + (nn + (long)r * n) * N::width;
+      double *bj = rhs + ((long)i * n + r) * N::width;
+      md::msum<N> sum;
+      sum.zero();
+      if (r < rows) {
+        if (part == 0) {
+          T v;
+          md::ldn(bj, v);
+          sum.set(v);
+        }
+        for (int l = part; l < n; l += 4) sum.fnma(ldn_at<N>(A, l), ldn_at<N>(x, l));
+      }
+      const T v = group4_sum<N>(sum.value());
+      if (r < rows && part == 0) md::stn(bj, v);
+    }
   }
   __syncthreads();
 }
