@@ -3,6 +3,7 @@
 // squares solve, one CTA per instance.
 #include "common.cuh"
 #include "dense.cuh"
+#include "tail_i8.cuh"
 
 namespace phc {
 
@@ -68,7 +69,7 @@ template <class N, bool OZ>
 __global__ void __launch_bounds__(kDenseThreads, 2)
     k_bals_solve(int n, int degp1, int szt, int tailidx, const double *__restrict__ mat, double *__restrict__ rhs,
                  double *__restrict__ sol, double *__restrict__ Q, double *__restrict__ Rm, int *__restrict__ flags,
-                 double *__restrict__ work, int stage) {
+                 double *__restrict__ work, int stage, int blocked) {
   extern __shared__ __align__(16) double sm[];
   typedef typename N::T T;
   const int W = N::width;
@@ -120,12 +121,31 @@ __global__ void __launch_bounds__(kDenseThreads, 2)
     for (int l = threadIdx.x; l < n; l += blockDim.x)
       stn_at<N>(S.x, l, ldn_at<N>(x, (long)(tail0 - 1) * n + l));
     __syncthreads();
+    unsigned active = 0;  // bit q mod 16: x of source stage q (x_{tail0-1+q}) is not skipped
     for (int i = tail0; i < degp1; ++i) {
+      // b_j -= A_{j-i+1} x_{i-1} for all j >= i; blocked: for the targets of
+      // the source's own block of four, the targets behind a block of 4, 8 or
+      // 16 sources together once the block is complete (block_tail_i8)
+      const int src = i - tail0;
       double nrm = warp_maxnorm<N>(n, S.x);
-      if (nrm < skip_tol<N>())
+      if (nrm < skip_tol<N>()) {
         ++up;
-      else
-        block_tail_update<N>(n, degp1, i, A, b, S.x);
+        active &= ~(1u << (src & 15));
+      } else {
+        active |= 1u << (src & 15);
+        block_tail_update<N>(n, blocked ? min(degp1, tail0 + (src | 3) + 1) : degp1, i, A, b, S.x);
+      }
+      if constexpr (N::tr::limbs == 4 && !N::is_complex) {
+        const int u = src + 1;
+        if (blocked && (u & 3) == 0) {
+          const int ns = (u & 15) == 0 ? 16 : ((u & 7) == 0 ? 8 : 4);
+          const int j0 = tail0 + u, j1 = ns == 16 ? degp1 : min(degp1, j0 + ns);
+          const unsigned mask = (active >> ((u - ns) & 15)) & ((1u << ns) - 1u);
+          if (j0 < j1 && mask)
+            block_tail_i8(n, A, b, x, tail0 - 1 + u - ns, ns, mask, j0, j1,
+                          reinterpret_cast<unsigned char *>(sm + dense_smem_doubles(n, szt, W)));
+        }
+      }
       const double *bi = b + (long)i * n * W;
       nrm = warp_maxnorm<N>(n, bi);
       double *xi = x + (long)i * n * W;
@@ -282,11 +302,16 @@ template <class N>
 static int bals_launch(int ninst, int n, int degp1, int szt, int tailidx, const double *mat, double *rhs, double *sol,
                        double *Q, double *R, int *flags, double *work, cudaStream_t st, bool oz) {
   const int stage = dense_stage(n, szt, N::width) ? 1 : 0;
-  const long smem = (stage ? dense_smem_doubles_staged(n, szt, N::width) : dense_smem_doubles(n, szt, N::width)) *
-                    (long)sizeof(double);
+  long smem = (stage ? dense_smem_doubles_staged(n, szt, N::width) : dense_smem_doubles(n, szt, N::width)) *
+              (long)sizeof(double);
+  // real quad-double of dimension 32..64 with a tail longer than one block of
+  // four: the digit products of tail_i8.cuh (their shared memory still lets
+  // two CTAs share an SM; the staged kernel has no room for it)
+  const int blocked = (N::tr::limbs == 4 && !N::is_complex && !stage && n >= kI8MinN && n <= kI8MaxN && degp1 > 5) ? 1 : 0;
+  if (blocked) smem += kI8Smem;
   auto kern = oz ? k_bals_solve<N, true> : k_bals_solve<N, false>;
   PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<ninst, kDenseThreads, smem, st>>>(n, degp1, szt, tailidx, mat, rhs, sol, Q, R, flags, work, stage);
+  kern<<<ninst, kDenseThreads, smem, st>>>(n, degp1, szt, tailidx, mat, rhs, sol, Q, R, flags, work, stage, blocked);
   PHC_CHECK_LAUNCH();
   return PHC_OK;
 }
