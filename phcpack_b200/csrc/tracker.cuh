@@ -469,6 +469,22 @@ __device__ __forceinline__ double warp_max_nonneg(double v) {
   return __hiloint2double((int)mhi, (int)mlo);
 }
 
+// X_ic <- X_ic + p F_ik (SUB: minus) for the rows i = i0, i0 + np, ... < end of
+// one column c of the row-major n x n matrix X, F_ik in column k of F (which
+// may be X); row ell reads q in place of X (an interchange).  (Three rows at
+// a time, loaded before any is stored, spilled: a path 25 % slower.)
+template <class N, bool SUB>
+__device__ __forceinline__ void column_update(int n, double *X, int c, const double *F, int k, int i0, int np, int end,
+                                              const typename N::T &p, int ell, const typename N::T &q) {
+  typedef typename N::T T;
+  #pragma unroll 1
+  for (int i = i0; i < end; i += np) {
+    const T x = (i == ell) ? q : ldn_at<N>(X, (long)i * n + c);
+    const T f = N::mul(p, ldn_at<N>(F, (long)i * n + k));
+    stn_at<N>(X, (long)i * n + c, SUB ? N::sub(x, f) : N::add(x, f));
+  }
+}
+
 // LU factorization with partial pivoting of the n x n matrix A (row-major,
 // shared memory, n <= 32), in place: lufac of
 // Math_Lib/Reduction/standard_complex_linear_solvers.adb:123-178 (LINPACK's
@@ -480,15 +496,16 @@ __device__ __forceinline__ double warp_max_nonneg(double v) {
 // CTA stay free).  Per column: lane i (k <= i < n) holds a_ik and forms its
 // reciprocal while the warp finds the largest candidate (warp_max_nonneg
 // and one ballot), so that 1 / a_kk is a shuffle away once the pivot row is
-// known; the rows swap (lanes over the columns); the (n-k-1)^2 entries of
-// the trailing update are spread over the lanes, each lane forming the
-// multiplier of its entry's row from column k; the multipliers are stored
-// last, a lane per row.  Every entry sees zgefa's operations in their order
-// (the results do not depend on the lane layout).  Called by all lanes of
-// the warp; returns info to every lane: 0, or k + 1 for the first column k
-// without a nonzero pivot.
+// known, and stores its multiplier.  The trailing update gives every column
+// j > k to 32 / (n-k-1) lanes that share its rows: each has read the two
+// entries of the swap before anything is written, so the swap costs no pass
+// of its own, and the pivot row's entry stays in a register; a factorization
+// is a chain of such columns, so what counts is the latency of one.  Every
+// entry sees zgefa's operations in their order (the results do not depend on
+// the lane layout).  Called by all lanes of the warp; returns info to every
+// lane: 0, or k + 1 for the first column k without a nonzero pivot.
 template <class N>
-__device__ TRACK_FN int warp_lufac(int n, double *A, int *ipvt, double *dinv) {
+__device__ __noinline__ int warp_lufac(int n, double *A, int *ipvt, double *dinv) {
   typedef typename N::T T;
   const int lane = threadIdx.x & 31;
   int info = 0;
@@ -517,39 +534,29 @@ __device__ TRACK_FN int warp_lufac(int n, double *A, int *ipvt, double *dinv) {
     }
     const T inv = md::shfl(r, ell);
     if (lane == 0) stn_at<N>(dinv, k, inv);
-    if (ell != k)
-      #pragma unroll 1
-      for (int j = k + lane; j < n; j += 32) {
-        const T t = ldn_at<N>(A, (long)ell * n + j);
-        stn_at<N>(A, (long)ell * n + j, ldn_at<N>(A, (long)k * n + j));
-        stn_at<N>(A, (long)k * n + j, t);
-      }
     // lane i's entry of column k after the swap (row ell holds the old row k)
     const T ak = md::shfl(a, k);
     const T ai = (lane == ell) ? ak : a;
     const T ninv = N::neg(inv);
-    __syncwarp();
-    // trailing update: entry (k+1+i, k+1+j) of the m x m block at e = i m + j
     const int m = n - k - 1;
-    if (m > 0) {
-      int i = lane / m, j = lane - (lane / m) * m;
-      const int qi = 32 / m, qj = 32 - (32 / m) * m;
-      #pragma unroll 1
-      for (int e = lane; e < m * m; e += 32) {
-        const long o = (long)(k + 1 + i) * n + (k + 1 + j);
-        const T mik = N::mul(ninv, ldn_at<N>(A, (long)(k + 1 + i) * n + k));
-        stn_at<N>(A, o, N::add(ldn_at<N>(A, o), N::mul(ldn_at<N>(A, (long)k * n + k + 1 + j), mik)));
-        i += qi;
-        j += qj;
-        if (j >= m) {
-          j -= m;
-          ++i;
-        }
-      }
+    const int np = m > 0 ? 32 / m : 1;  // lanes per column
+    const int part = m > 0 ? lane / m : 1;
+    const int j = k + 1 + lane - part * m;
+    const bool mine = part < np && m > 0;
+    T p = N::zero(), q = N::zero();  // rows ell and k of column j
+    if (mine) {
+      p = ldn_at<N>(A, (long)ell * n + j);
+      q = ldn_at<N>(A, (long)k * n + j);
     }
     __syncwarp();
-    // column k is not read again by this factorization
+    if (lane == ell && ell != k) stn_at<N>(A, (long)k * n + k, a);
     if (lane > k && lane < n) stn_at<N>(A, (long)lane * n + k, N::mul(ninv, ai));
+    __syncwarp();
+    if (mine) {
+      if (part == 0 && ell != k) stn_at<N>(A, (long)k * n + j, p);
+      column_update<N, false>(n, A, j, A, k, k + 1 + part, np, n, p, ell, q);
+    }
+    __syncwarp();
   }
   __syncwarp();
   return info;
@@ -588,68 +595,45 @@ __device__ typename N::T warp_lusolve(int n, const double *A, const int *ipvt, c
 }
 
 // M = A^{-1} from the factors of warp_lufac by one warp: lusolve applied to
-// the columns e_c of the identity, all columns at once, each substitution
-// step spread over the lanes (every entry sees the same operations in the
-// same order as a column-by-column solve; an entry's row and column follow
-// from the previous pass's by adding 32 = qi n + qc, without divisions).
-// Called by all lanes of one warp; the caller synchronises before M is read
-// by other warps.
+// the columns e_c of the identity, all columns at once.  A column belongs to
+// 32 / n lanes that share its rows; in each substitution step they first
+// read the step's entry (both entries of an interchange), then update their
+// rows (every entry sees the same operations in the same order as a
+// column-by-column solve).  Called by all lanes of one warp; the caller
+// synchronises before M is read by other warps.
 template <class N>
-__device__ TRACK_FN void warp_luinverse(int n, const double *A, const int *ipvt, const double *dinv, double *M) {
+__device__ __noinline__ void warp_luinverse(int n, const double *A, const int *ipvt, const double *dinv, double *M) {
   typedef typename N::T T;
   const int lane = threadIdx.x & 31;
-  const int i0 = lane / n, c0 = lane - (lane / n) * n;  // entry e = i n + c of lane's first pass
-  const int qi = 32 / n, qc = 32 - (32 / n) * n;
-  auto next = [&](int &i, int &c) {
-    i += qi;
-    c += qc;
-    if (c >= n) {
-      c -= n;
-      ++i;
-    }
-  };
-  {
-    int i = i0, c = c0;
+  const int np = 32 / n, part = lane / n, c = lane - part * n;
+  const bool mine = part < np;
+  if (mine)
     #pragma unroll 1
-    for (int e = lane; e < n * n; e += 32) {
-      stn_at<N>(M, e, (i == c) ? N::one() : N::zero());
-      next(i, c);
-    }
-  }
+    for (int i = part; i < n; i += np) stn_at<N>(M, (long)i * n + c, (i == c) ? N::one() : N::zero());
   __syncwarp();
   #pragma unroll 1
   for (int k = 0; k < n - 1; ++k) {  // L y = P e_c
     const int ell = ipvt[k];
-    if (ell != k)
-      #pragma unroll 1
-      for (int c = lane; c < n; c += 32) {
-        const T t = ldn_at<N>(M, (long)ell * n + c);
-        stn_at<N>(M, (long)ell * n + c, ldn_at<N>(M, (long)k * n + c));
-        stn_at<N>(M, (long)k * n + c, t);
-      }
+    T p = N::zero(), q = N::zero();
+    if (mine) {
+      p = ldn_at<N>(M, (long)ell * n + c);
+      q = ldn_at<N>(M, (long)k * n + c);
+    }
     __syncwarp();
-    const int m = n - k - 1;
-    int i = i0, c = c0;
-    #pragma unroll 1
-    for (int e = lane; e < m * n; e += 32) {
-      const long o = (long)(k + 1 + i) * n + c;
-      stn_at<N>(M, o, N::add(ldn_at<N>(M, o), N::mul(ldn_at<N>(M, (long)k * n + c), ldn_at<N>(A, (long)(k + 1 + i) * n + k))));
-      next(i, c);
+    if (mine) {
+      if (part == 0 && ell != k) stn_at<N>(M, (long)k * n + c, p);
+      column_update<N, false>(n, M, c, A, k, k + 1 + part, np, n, p, ell, q);
     }
     __syncwarp();
   }
   #pragma unroll 1
   for (int kb = n - 1; kb >= 0; --kb) {  // U x = y
-    #pragma unroll 1
-    for (int c = lane; c < n; c += 32)
-      stn_at<N>(M, (long)kb * n + c, N::mul(ldn_at<N>(M, (long)kb * n + c), ldn_at<N>(dinv, kb)));
+    T p = N::zero();
+    if (mine) p = N::mul(ldn_at<N>(M, (long)kb * n + c), ldn_at<N>(dinv, kb));
     __syncwarp();
-    int j = i0, c = c0;
-    #pragma unroll 1
-    for (int e = lane; e < kb * n; e += 32) {
-      const long o = (long)j * n + c;
-      stn_at<N>(M, o, N::sub(ldn_at<N>(M, o), N::mul(ldn_at<N>(M, (long)kb * n + c), ldn_at<N>(A, (long)j * n + kb))));
-      next(j, c);
+    if (mine) {
+      if (part == 0) stn_at<N>(M, (long)kb * n + c, p);
+      column_update<N, true>(n, M, c, A, kb, part, np, kb, p, -1, p);
     }
     __syncwarp();
   }
