@@ -138,17 +138,20 @@ __device__ TRACK_FN bool corrector_newton(const TrackDev &S, int s, int n, doubl
 // Resident CTAs per SM asked of the compiler (a register budget): 8 for the
 // precision-split tracker (double predictor, double-double refinement), whose
 // shared memory per path is small enough for 8 paths per SM; 1 otherwise.
-// The WIDE variant of the split tracker asks for one CTA fewer (72 registers
-// per thread instead of 64: fewer spills, each step a little faster); a batch
-// that fits on the GPU in one wave at that occupancy is launched with it.
-template <class PN, class RN, bool WIDE>
+// The variants of the split tracker with fewer CTAs have more registers (72
+// at 7, 128 at 4: fewer spills and more independent operations in flight, so
+// that a path's chain of steps is shorter); a batch that fits on the GPU in
+// one wave at a variant's occupancy is launched with it.
+template <class PN, class RN, int PER_SM>
 struct track_min_blocks {
   static const bool split = PN::width <= 2 && RN::width <= 4;
-  static const int value = split ? (WIDE ? TRACK_MINB - 1 : TRACK_MINB) : 1;
+  static const int value = split ? PER_SM : 1;
 };
+// PER_SM of the variants: the most paths per SM, one fewer, and few.
+static const int kTrackNarrow = TRACK_MINB, kTrackWide = TRACK_MINB - 1, kTrackFew = 4;
 
-template <class PN, class CN, class RN, bool WIDE>
-__global__ void __launch_bounds__(kTrackThreads, (track_min_blocks<PN, RN, WIDE>::value))
+template <class PN, class CN, class RN, int PER_SM>
+__global__ void __launch_bounds__(kTrackThreads, (track_min_blocks<PN, RN, PER_SM>::value))
     k_track(TrackDev S, TrackParDev P, int npaths, int path_begin, const int *__restrict__ path_sys,
             const double *__restrict__ x0, int *queue, const float *__restrict__ model, double *__restrict__ xend,
             int *__restrict__ info, double *__restrict__ dinfo, float *__restrict__ log, int log_cap,
@@ -546,7 +549,7 @@ static int track_launch(const TrackDev &S, const TrackParDev &P, int nmono_max, 
               nmono_max);
     return PHC_ERR_LIMIT;
   }
-  auto kern = k_track<PN, CN, RN, false>;
+  auto kern = k_track<PN, CN, RN, kTrackNarrow>;
   PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const float *mdl = reinterpret_cast<const float *>(model);
   if (one_per_launch) {
@@ -564,16 +567,28 @@ static int track_launch(const TrackDev &S, const TrackParDev &P, int nmono_max, 
   PHC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   PHC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kTrackThreads, smem));
   if (per < 1) per = 1;
-  if constexpr (track_min_blocks<PN, RN, true>::split) {
-    // one wave at the lower occupancy: take the variant with more registers
-    // (the autotuner's choice when it made one: 1 narrow, 2 wide)
-    auto wide = k_track<PN, CN, RN, true>;
+  const int cap = tune_get(kTuneTrackPerSM);
+  if constexpr (track_min_blocks<PN, RN, kTrackWide>::split) {
+    // one wave at a lower occupancy: take the variant with more registers
+    // (the autotuner's choice when it made one: 1 narrow, 2 wide).  On the
+    // dense quadratic n = 10 homotopy: 1024 paths 10.3 ms at 7 per SM against
+    // 12 ms at 4 (two waves); 500 paths 6.1 ms at 4 against 7.0 at 7; one
+    // path 3.5 against 4.1.
+    auto wide = k_track<PN, CN, RN, kTrackWide>;
+    auto few = k_track<PN, CN, RN, kTrackFew>;
     PHC_CUDA(cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_w = 0;
+    PHC_CUDA(cudaFuncSetAttribute(few, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_w = 0, per_f = 0;
     PHC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_w, wide, kTrackThreads, smem));
+    PHC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_f, few, kTrackThreads, smem));
     const int variant = tune_get(kTuneTrackVariant);
     const bool take_wide = variant == 2 || (variant == 0 && (long)npaths <= (long)nsm * per_w);
-    if (per_w >= 1 && take_wide) {
+    // paths per SM at once, when no more than the few-path variant can hold
+    const bool take_few = take_wide && ((long)npaths <= (long)nsm * per_f || (cap > 0 && cap <= per_f));
+    if (per_f >= 1 && take_few) {
+      kern = few;
+      per = per_f;
+    } else if (per_w >= 1 && take_wide) {
       kern = wide;
       per = per_w;
     }
@@ -581,7 +596,6 @@ static int track_launch(const TrackDev &S, const TrackParDev &P, int nmono_max, 
   // paths tracked at once per SM: all the resident CTAs the occupancy allows,
   // or fewer when the autotuner found that faster (fewer paths share an SM's
   // issue slots; the work queue hands the rest out as paths finish)
-  const int cap = tune_get(kTuneTrackPerSM);
   if (cap > 0 && cap < per) per = cap;
   long grid = (long)nsm * per;
   if (grid > npaths) grid = npaths;
