@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(kTrackThreads, 1)
   const int n = S.dim[s];
   const double t = tpt[path];
   const int lane = ctid() & 31, warp = ctid() >> 5;
+  mono_table(S, s, sm + L.hbuf);
   // the point, its limbs truncated or padded to the working precision
   double *xc = sm + L.xc;
   for (int q = ctid(); q < n * Wp; q += blockDim.x) {

@@ -95,6 +95,37 @@ __host__ __device__ inline bool simple_monomial(int k, const int *ex) {
   return (k == 1 && ex[0] >= 1 && ex[0] <= 2) || (k == 2 && ex[0] == 1 && ex[1] == 1);
 }
 
+// A monomial's kind and variables in one word: kMonoOne the constant 1,
+// kMonoVar x_i, kMonoProd x_i x_l (l = i for a square), kMonoOther any
+// other; i in bits 0..4, l in bits 5..9, the kind from bit 10.
+enum { kMonoOther = 0, kMonoOne = 1, kMonoVar = 2, kMonoProd = 3 };
+__device__ __forceinline__ unsigned mono_encode(const TrackDev &S, int gm) {
+  const int k = S.mono_nvr[gm];
+  const int *ix = S.mono_idx + (long)gm * S.maxvar;
+  const int *ex = S.mono_exp + (long)gm * S.maxvar;
+  if (k == 0) return kMonoOne << 10;
+  if (!simple_monomial(k, ex)) return kMonoOther << 10;
+  if (k == 1 && ex[0] == 1) return (kMonoVar << 10) | (unsigned)ix[0];
+  return (kMonoProd << 10) | ((unsigned)(k == 2 ? ix[1] : ix[0]) << 5) | (unsigned)ix[0];
+}
+// The words of the system's first kMonoTable monomials in shared memory,
+// formed once per path: every evaluation reads a word instead of a chain of
+// three dependent loads of supports.  They lie in the half of the network's
+// activation buffer (TrackLayout::hbuf) that the network leaves unused.
+static const int kMonoTable = 528;
+__shared__ unsigned short *track_mono;
+__device__ __forceinline__ unsigned mono_word(const TrackDev &S, int m0, int m) {
+  return m < kMonoTable ? (unsigned)track_mono[m] : mono_encode(S, m0 + m);
+}
+// Called by all threads; the caller synchronises before the first use.
+__device__ __forceinline__ void mono_table(const TrackDev &S, int s, double *hbuf) {
+  unsigned short *t = reinterpret_cast<unsigned short *>(hbuf) + kMonoTable;
+  const int m0 = S.mono_off[s], nm = S.mono_off[s + 1] - m0;
+  if (ctid() == 0) track_mono = t;
+  #pragma unroll 1
+  for (int m = ctid(); m < nm && m < kMonoTable; m += blockDim.x) t[m] = (unsigned short)mono_encode(S, m0 + m);
+}
+
 // Tracking parameters (include/phc_b200.h, phc_track: ipar and dpar)
 struct TrackParDev {
   int deg, numdeg, dendeg, nit, corsteps, maxsteps, refine_steps, step_mode;
@@ -202,15 +233,13 @@ __device__ TRACK_FN void hom_eval_cta(const TrackDev &S, int s, int w, double t0
   #pragma unroll 1
   for (int m = ctid(); m < nm; m += blockDim.x) {
     const int gm = m0 + m;
-    const int k = S.mono_nvr[gm];
-    const int *ix = S.mono_idx + (long)gm * mv;
-    const int *ex = S.mono_exp + (long)gm * mv;
-    if (k >= 1 && simple_monomial(k, ex)) {
+    const unsigned word = mono_word(S, m0, m);
+    if ((word >> 10) >= kMonoVar) {
       // value only: x_j, x_j^2 or x_j x_l (the partials are read in place)
       double *Vm = V + (long)m * n1 * W;
-      const double *xa = x + (long)ix[0] * xld * W;
-      const double *xb = (k == 2) ? x + (long)ix[1] * xld * W : xa;
-      if (k == 1 && ex[0] == 1) {
+      const double *xa = x + (long)(word & 31) * xld * W;
+      const double *xb = x + (long)((word >> 5) & 31) * xld * W;
+      if ((word >> 10) == kMonoVar) {
         #pragma unroll 1
         for (int i = 0; i < n1; ++i) stn_at<N>(Vm, i, ldn_at<N>(xa, i));
       } else {
@@ -224,6 +253,9 @@ __device__ TRACK_FN void hom_eval_cta(const TrackDev &S, int s, int w, double t0
       }
       continue;
     }
+    const int k = S.mono_nvr[gm];
+    const int *ix = S.mono_idx + (long)gm * mv;
+    const int *ex = S.mono_exp + (long)gm * mv;
     T F[kTrackKmax + 1], acc[kTrackKmax + 1];
     bool unitF = true;
     #pragma unroll 1
@@ -391,49 +423,49 @@ __device__ TRACK_FN void hom_coef_cta(const TrackDev &S, int s, int k, double t0
   const int m0 = S.mono_off[s];
   const int nm = S.mono_off[s + 1] - m0;
   const int mv = S.maxvar;
+  // items: the coefficients k of the monomials, then the coefficients k - 1
+  // (in reverse, so that a thread's second item is one of the constant and
+  // linear monomials, which come first)
   #pragma unroll 1
-  for (int m = ctid(); m < nm; m += blockDim.x) {
-    const int gm = m0 + m;
-    const int kv = S.mono_nvr[gm];
-    const int *ix = S.mono_idx + (long)gm * mv;
-    const int *ex = S.mono_exp + (long)gm * mv;
-    T c1 = N::zero(), c2 = N::zero();  // coefficients k-1 and k
-    if (kv == 0) {
-      if (k == 1) c1 = N::one();
-    } else if (simple_monomial(kv, ex)) {
-      const double *xa = x + (long)ix[0] * xld * W;
-      const double *xb = (kv == 2) ? x + (long)ix[1] * xld * W : xa;
-      if (kv == 1 && ex[0] == 1) {
-        c1 = ldn_at<N>(xa, k - 1);
-        c2 = ldn_at<N>(xa, k);
-      } else {
-        #pragma unroll 1
-        for (int i = 0; i <= k - 1; ++i) c1 = N::add(c1, N::mul(ldn_at<N>(xa, i), ldn_at<N>(xb, k - 1 - i)));
-        #pragma unroll 1
-        for (int i = 0; i <= k; ++i) c2 = N::add(c2, N::mul(ldn_at<N>(xa, i), ldn_at<N>(xb, k - i)));
-      }
+  for (int it = ctid(); it < 2 * nm; it += blockDim.x) {
+    const int hi = it < nm ? 1 : 0;
+    const int m = hi ? it : 2 * nm - 1 - it;
+    const int kc = k - 1 + hi;
+    const unsigned word = mono_word(S, m0, m), kind = word >> 10;
+    T c = N::zero();
+    if (kind == kMonoOne) {
+      if (kc == 0) c = N::one();
+    } else if (kind == kMonoVar) {
+      c = ldn_at<N>(x, (long)(word & 31) * xld + kc);
+    } else if (kind == kMonoProd) {
+      const double *xa = x + (long)(word & 31) * xld * W;
+      const double *xb = x + ((long)((word >> 5) & 31) * xld + kc) * W;
+      #pragma unroll 1
+      for (int i = 0; i <= kc; ++i, xa += W, xb -= W) c = N::add(c, N::mul(ldn_at<N>(xa, 0), ldn_at<N>(xb, 0)));
     } else {
+      const int gm = m0 + m;
+      const int kv = S.mono_nvr[gm];
+      const int *ix = S.mono_idx + (long)gm * mv;
+      const int *ex = S.mono_exp + (long)gm * mv;
       T F[kTrackKmax + 1];
       #pragma unroll 1
-      for (int i = 0; i <= k; ++i) F[i] = (i == 0) ? N::one() : N::zero();
+      for (int i = 0; i <= kc; ++i) F[i] = (i == 0) ? N::one() : N::zero();
       #pragma unroll 1
       for (int v = 0; v < kv; ++v)
         #pragma unroll 1
         for (int e = 0; e < ex[v]; ++e) {
           const double *xv = x + (long)ix[v] * xld * W;
           #pragma unroll 1
-          for (int kk = k; kk >= 0; --kk) {  // in place: F[kk] only needs F[<= kk]
+          for (int kk = kc; kk >= 0; --kk) {  // in place: F[kk] only needs F[<= kk]
             T a = N::zero();
             #pragma unroll 1
             for (int i = 0; i <= kk; ++i) a = N::add(a, N::mul(ldn_at<N>(xv, i), F[kk - i]));
             F[kk] = a;
           }
         }
-      c1 = F[k - 1];
-      c2 = F[k];
+      c = F[kc];
     }
-    stn_at<N>(V2, 2L * m, c1);
-    stn_at<N>(V2, 2L * m + 1, c2);
+    stn_at<N>(V2, 2L * m + hi, c);
   }
   __syncthreads();
   const int e0 = S.eq_off[s];
@@ -1243,20 +1275,11 @@ __device__ TRACK_FN bool point_newton_split(const TrackDev &S, int s, int n, dou
     // the distinct monomials x^e in double-double, one per thread
     #pragma unroll 1
     for (int m = ctid(); m < nm; m += kTrackThreads) {
-      const int gm = m0 + m;
-      const int nv = S.mono_nvr[gm];
-      const int *ix = S.mono_idx + (long)gm * S.maxvar;
-      const int *ex = S.mono_exp + (long)gm * S.maxvar;
+      const unsigned word = mono_word(S, m0, m), kind = word >> 10;
       T v = N::one();
-      bool unit = true;
-      #pragma unroll 1
-      for (int u = 0; u < nv; ++u) {
-        const T xu = ldn_at<N>(x, ix[u]);
-        #pragma unroll 1
-        for (int q = 0; q < ex[u]; ++q) {
-          v = unit ? xu : N::mul(v, xu);
-          unit = false;
-        }
+      if (kind >= kMonoVar) {
+        v = ldn_at<N>(x, word & 31);
+        if (kind == kMonoProd) v = N::mul(v, ldn_at<N>(x, (word >> 5) & 31));
       }
       stn_at<N>(V, m, v);
     }

@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(kTrackThreads, (track_min_blocks<PN, RN, PER_S
     const int s = path_sys[path];
     const int n = S.dim[s];
     double *xc = sm + L.xc;
+    mono_table(S, s, sm + L.hbuf);
     // start point, refined at t = 0
     #pragma unroll 1
     for (int i = ctid(); i < n; i += blockDim.x) {
