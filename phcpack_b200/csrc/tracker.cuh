@@ -447,16 +447,27 @@ __device__ TRACK_FN void hom_coef_cta(const TrackDev &S, int s, int k, double t0
       const int kv = S.mono_nvr[gm];
       const int *ix = S.mono_idx + (long)gm * mv;
       const int *ex = S.mono_exp + (long)gm * mv;
+      // the product of its d factors: the first series is read in place of a
+      // product with 1, the last factor's product needs coefficient kc alone
+      // (the same operations on the same numbers as all coefficients of all
+      // products; a cubic's Taylor steps were 60 % of its tracking time)
       T F[kTrackKmax + 1];
+      int d = 0;
       #pragma unroll 1
-      for (int i = 0; i <= kc; ++i) F[i] = (i == 0) ? N::one() : N::zero();
+      for (int v = 0; v < kv; ++v) d += ex[v];
+      int f = 0;  // factors taken
       #pragma unroll 1
       for (int v = 0; v < kv; ++v)
         #pragma unroll 1
-        for (int e = 0; e < ex[v]; ++e) {
+        for (int e = 0; e < ex[v]; ++e, ++f) {
           const double *xv = x + (long)ix[v] * xld * W;
+          if (f == 0) {
+            #pragma unroll 1
+            for (int i = 0; i <= kc; ++i) F[i] = ldn_at<N>(xv, i);
+            continue;
+          }
           #pragma unroll 1
-          for (int kk = kc; kk >= 0; --kk) {  // in place: F[kk] only needs F[<= kk]
+          for (int kk = kc; kk >= (f == d - 1 ? kc : 0); --kk) {  // in place: F[kk] only needs F[<= kk]
             T a = N::zero();
             #pragma unroll 1
             for (int i = 0; i <= kk; ++i) a = N::add(a, N::mul(ldn_at<N>(xv, i), F[kk - i]));
@@ -500,6 +511,11 @@ __device__ __forceinline__ double warp_max_nonneg(double v) {
   const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);
   return __hiloint2double((int)mhi, (int)mlo);
 }
+
+// ceil(2^16 / m): (x * small_inverse[m]) >> 16 = x / m for 0 <= x <= 32
+__constant__ int small_inverse[33] = {
+    0,    65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192, 7282, 6554, 5958, 5462, 5042, 4682, 4370, 4096,
+    3856, 3641,  3450,  3277,  3121,  2979,  2850,  2731, 2622, 2521, 2428, 2341, 2260, 2185, 2115, 2048};
 
 // X_ic <- X_ic + p F_ik (SUB: minus) for the rows i = i0, i0 + np, ... < end of
 // one column c of the row-major n x n matrix X, F_ik in column k of F (which
@@ -552,13 +568,22 @@ __device__ __noinline__ int warp_lufac(int n, double *A, int *ipvt, double *dinv
       if (!(v == v)) v = INFINITY;  // a NaN pivot candidate reads as infinity
     }
     const T r = cand ? N::div(N::one(), a) : N::zero();
-    // the largest value, then the first row that holds it (one ballot)
-    const double mx = warp_max_nonneg(v);
-    const unsigned hold = __ballot_sync(0xffffffffu, cand && v == mx);
-    const int ix = hold ? __ffs(hold) - 1 : n;
-    const int ell = ix < n ? ix : n - 1;
+    // the first row of the largest value: by the high words alone when one
+    // row holds the largest, by the whole values otherwise
+    const unsigned hi = cand ? (unsigned)__double2hiint(v) : 0u;
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+    unsigned hold = __ballot_sync(0xffffffffu, cand && hi == mhi);
+    bool zero = false;
+    if (hold & (hold - 1)) {
+      const double mx = warp_max_nonneg(v);
+      hold = __ballot_sync(0xffffffffu, cand && v == mx);
+      zero = mx == 0.0;
+    } else if (mhi == 0u) {
+      zero = __shfl_sync(0xffffffffu, v, __ffs(hold) - 1) == 0.0;
+    }
+    const int ell = __ffs(hold) - 1;
     if (lane == 0) ipvt[k] = ell;
-    if (mx == 0.0) {
+    if (zero) {
       if (info == 0) info = k + 1;  // this column is already triangularized
       if (lane == 0) stn_at<N>(dinv, k, N::from(NAN));
       __syncwarp();
@@ -571,8 +596,9 @@ __device__ __noinline__ int warp_lufac(int n, double *A, int *ipvt, double *dinv
     const T ai = (lane == ell) ? ak : a;
     const T ninv = N::neg(inv);
     const int m = n - k - 1;
-    const int np = m > 0 ? 32 / m : 1;  // lanes per column
-    const int part = m > 0 ? lane / m : 1;
+    const int inv_m = small_inverse[m];
+    const int np = m > 0 ? (32 * inv_m) >> 16 : 1;  // lanes per column: 32 / m
+    const int part = m > 0 ? (lane * inv_m) >> 16 : 1;  // lane / m
     const int j = k + 1 + lane - part * m;
     const bool mine = part < np && m > 0;
     T p = N::zero(), q = N::zero();  // rows ell and k of column j
@@ -608,20 +634,28 @@ __device__ typename N::T warp_lusolve(int n, const double *A, const int *ipvt, c
   // lane k's reciprocal pivot dinv[k], read once before the substitutions
   // (off the dependent chain of the back substitution)
   const T dl = (lane < n) ? ldn_at<N>(dinv, lane) : N::zero();
+  // lane k's row interchange; each step's column entry is loaded a step ahead
+  const int pl = lane < n ? ipvt[lane] : 0;
+  const double *row = A + (long)(lane < n ? lane : 0) * n * N::width;
+  T f = ldn_at<N>(row, 0);
   #pragma unroll 1
   for (int k = 0; k < n - 1; ++k) {  // L y = P b
-    const int ell = ipvt[k];
+    const T fn = ldn_at<N>(row, k + 1);
+    const int ell = __shfl_sync(0xffffffffu, pl, k);
     const T t = md::shfl(v, ell);
     const T bk = md::shfl(v, k);
     if (lane == ell) v = bk;
     if (lane == k) v = t;
-    if (lane > k && lane < n) v = N::add(v, N::mul(t, ldn_at<N>(A, (long)lane * n + k)));
+    if (lane > k && lane < n) v = N::add(v, N::mul(t, f));
+    f = fn;
   }
   #pragma unroll 1
-  for (int kb = n - 1; kb >= 0; --kb) {  // U x = y
+  for (int kb = n - 1; kb >= 0; --kb) {  // U x = y (f: column kb)
+    const T fn = ldn_at<N>(row, kb > 0 ? kb - 1 : 0);
     if (lane == kb) v = N::mul(v, dl);
     const T t = md::shfl(v, kb);
-    if (lane < kb) v = N::sub(v, N::mul(t, ldn_at<N>(A, (long)lane * n + kb)));
+    if (lane < kb) v = N::sub(v, N::mul(t, f));
+    f = fn;
   }
   return v;
 }
@@ -1258,15 +1292,28 @@ __device__ TRACK_FN bool point_newton_split(const TrackDev &S, int s, int n, dou
       const int i = e / n, j = e % n;
       const int g = (e0 + i) * S.maxdim + j;
       double2 acc = make_double2(0.0, 0.0);
+      const int qe = S.jg_off[g + 1];
+      int q = S.jg_off[g];
+      int tr = 0, sl = -1;
+      if (q < qe) {
+        tr = S.jg_term[q];
+        sl = S.jg_slot[q];
+      }
       #pragma unroll 1
-      for (int q = S.jg_off[g]; q < S.jg_off[g + 1]; ++q) {
-        const int tr = S.jg_term[q], sl = S.jg_slot[q];
+      for (; q < qe; ++q) {
         const double ar = S.term_a[2 * tr], ai = S.term_a[2 * tr + 1];
-        const double2 c = make_double2(fma(S.term_b[2 * tr] - ar, t, ar), fma(S.term_b[2 * tr + 1] - ai, t, ai));
-        double2 v;
-        if (sl == -1) v = make_double2(1.0, 0.0);
-        else if (sl == -2) v = make_double2(2.0 * xj[j].x, 2.0 * xj[j].y);
-        else v = xj[-sl - 3];
+        const double br = S.term_b[2 * tr], bi = S.term_b[2 * tr + 1];
+        // the constant 1, 2 x_j or x_l, without branches
+        double2 v = xj[sl <= -3 ? -sl - 3 : j];
+        const int sc = sl;
+        if (q + 1 < qe) {  // the next entry, ahead of this one's operations
+          tr = S.jg_term[q + 1];
+          sl = S.jg_slot[q + 1];
+        }
+        const double2 c = make_double2(fma(br - ar, t, ar), fma(bi - ai, t, ai));
+        const double f = sc == -2 ? 2.0 : 1.0;
+        v.x = sc == -1 ? 1.0 : f * v.x;
+        v.y = sc == -1 ? 0.0 : f * v.y;
         acc.x = fma(c.x, v.x, fma(-c.y, v.y, acc.x));
         acc.y = fma(c.x, v.y, fma(c.y, v.x, acc.y));
       }
