@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(kTrackThreads, 1)
     for (int k = 1; k <= K; ++k) {
       hom_coef_cta<PN>(S, s, k, t, xs, K + 1, sm + L.V, sm + L.r);
       for (int i = ctid(); i < n; i += blockDim.x) {
-        T acc = PN::zero();
-        for (int j = 0; j < n; ++j)
-          acc = PN::add(acc, PN::mul(ldn_at<PN>(sm + L.M, (long)i * n + j), ldn_at<PN>(sm + L.r, j)));
-        stn_at<PN>(xs, (long)i * (K + 1) + k, PN::neg(acc));
+        term_sum<PN> acc;
+        acc.zero();
+        for (int j = 0; j < n; ++j) acc.fma(ldn_at<PN>(sm + L.M, (long)i * n + j), ldn_at<PN>(sm + L.r, j));
+        stn_at<PN>(xs, (long)i * (K + 1) + k, PN::neg(acc.value()));
       }
       __syncthreads();
     }

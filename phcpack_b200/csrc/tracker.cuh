@@ -193,6 +193,22 @@ template <> struct conv_num<md::num<md::qd, true>, md::num<md::dd, true> > {
   }
 };
 
+// Sum of products a b in the tracker's evaluations.  In double every product
+// and every sum is rounded by itself (the step decisions rest on these
+// numbers); in the multiple-double precisions the products go into the open
+// accumulators of md::msum: fewer operations, and one addition instead of
+// some thirty dependent operations from one term to the next, which is what
+// a path's chain is made of.
+template <class N, bool PLAIN = N::tr::limbs == 1 || (N::tr::limbs > 4)>
+struct term_sum {
+  typename N::T a;
+  __device__ __forceinline__ void zero() { a = N::zero(); }
+  __device__ __forceinline__ void fma(const typename N::T &x, const typename N::T &y) { a = N::add(a, N::mul(x, y)); }
+  __device__ __forceinline__ typename N::T value() const { return a; }
+};
+template <class N>
+struct term_sum<N, false> : md::msum<N> {};
+
 template <class N>
 __device__ __forceinline__ typename N::T cnum(double re, double im) {
   typename N::T r = N::from(re);
@@ -328,9 +344,9 @@ __device__ TRACK_FN void hom_eval_cta(const TrackDev &S, int s, int w, double t0
     const int tb = S.term_off[e0 + i], te = S.term_off[e0 + i + 1];
     #pragma unroll 1
     for (int k0 = 0; k0 < n1; k0 += KC) {
-      T acc[KC];
+      term_sum<N> acc[KC];
 #pragma unroll
-      for (int r = 0; r < KC; ++r) acc[r] = N::zero();
+      for (int r = 0; r < KC; ++r) acc[r].zero();
       #pragma unroll 1
       for (int tr = tb + lane; tr < te; tr += 32) {
         const T a = cnum<N>(S.term_a[2 * tr], S.term_a[2 * tr + 1]);
@@ -343,8 +359,8 @@ __device__ TRACK_FN void hom_eval_cta(const TrackDev &S, int s, int w, double t0
           const int kk = k0 + r;
           if (kk < n1) {
             const T v = ldn_at<N>(Vm, kk);
-            acc[r] = N::add(acc[r], N::mul(c0, v));
-            if (kk > 0) acc[r] = N::add(acc[r], N::mul(b, prev));
+            acc[r].fma(c0, v);
+            if (kk > 0) acc[r].fma(b, prev);
             prev = v;
           }
         }
@@ -352,7 +368,7 @@ __device__ TRACK_FN void hom_eval_cta(const TrackDev &S, int s, int w, double t0
 #pragma unroll
       for (int r = 0; r < KC; ++r)
         if (k0 + r < n1) {
-          const T sum = warp_sum<N>(acc[r]);
+          const T sum = warp_sum<N>(acc[r].value());
           if (lane == 0) stn_at<N>(h, (long)i * n1 + k0 + r, sum);
         }
     }
@@ -365,9 +381,9 @@ __device__ TRACK_FN void hom_eval_cta(const TrackDev &S, int s, int w, double t0
       const int qb = S.jg_off[g], qe = S.jg_off[g + 1];
       #pragma unroll 1
       for (int k0 = 0; k0 < n1; k0 += KC) {
-        JT acc[KC];
+        term_sum<JN> acc[KC];
 #pragma unroll
-        for (int r = 0; r < KC; ++r) acc[r] = JN::zero();
+        for (int r = 0; r < KC; ++r) acc[r].zero();
         #pragma unroll 1
         for (int q = qb; q < qe; ++q) {
           const int tr = S.jg_term[q];
@@ -391,15 +407,15 @@ __device__ TRACK_FN void hom_eval_cta(const TrackDev &S, int s, int w, double t0
             const int kk = k0 + r;
             if (kk < n1) {
               const JT v = gload(kk);
-              acc[r] = JN::add(acc[r], JN::mul(c0, v));
-              if (kk > 0) acc[r] = JN::add(acc[r], JN::mul(b, prev));
+              acc[r].fma(c0, v);
+              if (kk > 0) acc[r].fma(b, prev);
               prev = v;
             }
           }
         }
 #pragma unroll
         for (int r = 0; r < KC; ++r)
-          if (k0 + r < n1) stn_at<JN>(J, ((long)(k0 + r) * n + i) * n + j, acc[r]);
+          if (k0 + r < n1) stn_at<JN>(J, ((long)(k0 + r) * n + i) * n + j, acc[r].value());
       }
     }
   }
@@ -440,8 +456,11 @@ __device__ TRACK_FN void hom_coef_cta(const TrackDev &S, int s, int k, double t0
     } else if (kind == kMonoProd) {
       const double *xa = x + (long)(word & 31) * xld * W;
       const double *xb = x + ((long)((word >> 5) & 31) * xld + kc) * W;
+      term_sum<N> sum;
+      sum.zero();
       #pragma unroll 1
-      for (int i = 0; i <= kc; ++i, xa += W, xb -= W) c = N::add(c, N::mul(ldn_at<N>(xa, 0), ldn_at<N>(xb, 0)));
+      for (int i = 0; i <= kc; ++i, xa += W, xb -= W) sum.fma(ldn_at<N>(xa, 0), ldn_at<N>(xb, 0));
+      c = sum.value();
     } else {
       const int gm = m0 + m;
       const int kv = S.mono_nvr[gm];
@@ -468,10 +487,11 @@ __device__ TRACK_FN void hom_coef_cta(const TrackDev &S, int s, int k, double t0
           }
           #pragma unroll 1
           for (int kk = kc; kk >= (f == d - 1 ? kc : 0); --kk) {  // in place: F[kk] only needs F[<= kk]
-            T a = N::zero();
+            term_sum<N> sum;
+            sum.zero();
             #pragma unroll 1
-            for (int i = 0; i <= kk; ++i) a = N::add(a, N::mul(ldn_at<N>(xv, i), F[kk - i]));
-            F[kk] = a;
+            for (int i = 0; i <= kk; ++i) sum.fma(ldn_at<N>(xv, i), F[kk - i]);
+            F[kk] = sum.value();
           }
         }
       c = F[kc];
@@ -483,17 +503,18 @@ __device__ TRACK_FN void hom_coef_cta(const TrackDev &S, int s, int k, double t0
   const int lane = ctid() & 31, warp = ctid() >> 5, nw = blockDim.x >> 5;
   #pragma unroll 1
   for (int i = warp; i < n; i += nw) {
-    T acc = N::zero();
+    term_sum<N> sum;
+    sum.zero();
     #pragma unroll 1
     for (int tr = S.term_off[e0 + i] + lane; tr < S.term_off[e0 + i + 1]; tr += 32) {
       const T a = cnum<N>(S.term_a[2 * tr], S.term_a[2 * tr + 1]);
       const T b = N::sub(cnum<N>(S.term_b[2 * tr], S.term_b[2 * tr + 1]), a);  // d/dt
       const T c0 = N::add(a, N::scale_d(b, t0));
       const long mm = 2L * (S.term_mono[tr] - m0);
-      acc = N::add(acc, N::mul(c0, ldn_at<N>(V2, mm + 1)));
-      acc = N::add(acc, N::mul(b, ldn_at<N>(V2, mm)));
+      sum.fma(c0, ldn_at<N>(V2, mm + 1));
+      sum.fma(b, ldn_at<N>(V2, mm));
     }
-    acc = warp_sum<N>(acc);
+    const T acc = warp_sum<N>(sum.value());
     if (lane == 0) stn_at<N>(r, i, acc);
   }
   __syncthreads();

@@ -267,11 +267,11 @@ __global__ void __launch_bounds__(kTrackThreads, (track_min_blocks<PN, RN, PER_S
         hom_coef_cta<PN>(S, s, k, t, xs, K + 1, sm + L.V, sm + L.r);
         #pragma unroll 1
         for (int i = ctid(); i < n; i += blockDim.x) {
-          typename PN::T acc = PN::zero();
+          term_sum<PN> acc;
+          acc.zero();
           #pragma unroll 1
-          for (int j = 0; j < n; ++j)
-            acc = PN::add(acc, PN::mul(ldn_at<PN>(sm + L.M, (long)i * n + j), ldn_at<PN>(sm + L.r, j)));
-          stn_at<PN>(xs, (long)i * (K + 1) + k, PN::neg(acc));
+          for (int j = 0; j < n; ++j) acc.fma(ldn_at<PN>(sm + L.M, (long)i * n + j), ldn_at<PN>(sm + L.r, j));
+          stn_at<PN>(xs, (long)i * (K + 1) + k, PN::neg(acc.value()));
         }
         __syncthreads();
       }
