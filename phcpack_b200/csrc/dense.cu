@@ -15,8 +15,19 @@ __host__ __device__ inline long dense_stride(int n, int szt, int W, bool oz) {
   return dense_work_numbers(n, szt) * W + (oz ? ozaki_work_doubles(n, ozaki_slices<md::qd>::s) : 0);
 }
 
-template <class N, bool OZ>
-__global__ void __launch_bounds__(kDenseThreads, 2)
+// CTAs per SM asked of the compiler (a register budget).  A batch that gives
+// every SM more than two instances wants many (dimension 60, tile 10, degree
+// 31, 512 instances: double 4.8 ms at two per SM, 2.9 at four; double-double
+// 7.1 and 5.0), a smaller one registers (100 instances of dimension 48,
+// double-double: 2.1 ms at two, 2.3 at four); quad-double needs 128 registers.
+template <class N>
+struct dense_many {
+  static const int value = N::tr::limbs == 1 ? 4 : (N::tr::limbs == 2 ? (N::is_complex ? 3 : 4) : 2);
+};
+static const int kDenseFew = 2;
+
+template <class N, bool OZ, int PER_SM>
+__global__ void __launch_bounds__(kDenseThreads, PER_SM)
     k_blocked_houseqr(int n, int ncols, int szt, const double *__restrict__ A, double *__restrict__ Q,
                       double *__restrict__ Rm, double *__restrict__ work, int stage) {
   extern __shared__ __align__(16) double sm[];
@@ -39,7 +50,7 @@ __global__ void __launch_bounds__(kDenseThreads, 2)
 // overwritten by the updated right hand sides and the diagonal tiles of U by
 // their inverses.
 template <class N>
-__global__ void __launch_bounds__(kDenseThreads, 2)
+__global__ void __launch_bounds__(kDenseThreads, dense_many<N>::value)
     k_upper_tiled_solver(int dim, int szt, double *__restrict__ U, double *__restrict__ b, double *__restrict__ x,
                          double *__restrict__ work) {
   const int W = N::width;
@@ -65,8 +76,8 @@ __global__ void __launch_bounds__(kDenseThreads, 2)
 // right hand side below 1e-28; 1e-15 and 1e-56 in double and quad-double).
 // flags per instance: zeroQ, noqr, upidx, bsidx, newtail; with tailidx < 0
 // the tail starts at the instance's flags[4].
-template <class N, bool OZ>
-__global__ void __launch_bounds__(kDenseThreads, 2)
+template <class N, bool OZ, int PER_SM>
+__global__ void __launch_bounds__(kDenseThreads, PER_SM)
     k_bals_solve(int n, int degp1, int szt, int tailidx, const double *__restrict__ mat, double *__restrict__ rhs,
                  double *__restrict__ sol, double *__restrict__ Q, double *__restrict__ Rm, int *__restrict__ flags,
                  double *__restrict__ work, int stage, int blocked) {
@@ -189,13 +200,27 @@ static bool dense_stage(int n, int szt, int W) {
   return tune_get(kTuneDenseStage) == 2 && staged <= 227L * 1024 - 1024;
 }
 
+// More than two instances per SM of the current device?
+static int dense_wants_many(int ninst, bool *many) {
+  int dev = 0, nsm = 148;
+  PHC_CUDA(cudaGetDevice(&dev));
+  PHC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  *many = (long)ninst > (long)kDenseFew * nsm;
+  return PHC_OK;
+}
+
 template <class N>
 static int qr_launch(int ninst, int n, int ncols, int szt, const double *A, double *Q, double *R, double *work,
                      cudaStream_t st, bool oz) {
   const int stage = dense_stage(n, szt, N::width) ? 1 : 0;
   const long smem = (stage ? dense_smem_doubles_staged(n, szt, N::width) : dense_smem_doubles(n, szt, N::width)) *
                     (long)sizeof(double);
-  auto kern = oz ? k_blocked_houseqr<N, true> : k_blocked_houseqr<N, false>;
+  bool many = false;
+  const int rc = dense_wants_many(ninst, &many);
+  if (rc) return rc;
+  const int kMany = dense_many<N>::value;
+  auto kern = oz ? (many ? k_blocked_houseqr<N, true, kMany> : k_blocked_houseqr<N, true, kDenseFew>)
+                 : (many ? k_blocked_houseqr<N, false, kMany> : k_blocked_houseqr<N, false, kDenseFew>);
   PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<ninst, kDenseThreads, smem, st>>>(n, ncols, szt, A, Q, R, work, stage);
   PHC_CHECK_LAUNCH();
@@ -225,7 +250,7 @@ __device__ __forceinline__ void residue_dec(typename N::T &r, const typename N::
 }
 
 template <class N>
-__global__ void __launch_bounds__(kDenseThreads, 2)
+__global__ void __launch_bounds__(kDenseThreads)
     k_linear_residue(int n, int degp1, int tailidx, const double *__restrict__ mat, const double *__restrict__ rhs,
                      const double *__restrict__ sol, double *__restrict__ res, double *__restrict__ resmax) {
   typedef typename N::T T;
@@ -309,7 +334,12 @@ static int bals_launch(int ninst, int n, int degp1, int szt, int tailidx, const 
   // two CTAs share an SM; the staged kernel has no room for it)
   const int blocked = (N::tr::limbs == 4 && !N::is_complex && !stage && n >= kI8MinN && n <= kI8MaxN && degp1 > 5) ? 1 : 0;
   if (blocked) smem += kI8Smem;
-  auto kern = oz ? k_bals_solve<N, true> : k_bals_solve<N, false>;
+  bool many = false;
+  const int rc = dense_wants_many(ninst, &many);
+  if (rc) return rc;
+  const int kMany = dense_many<N>::value;
+  auto kern = oz ? (many ? k_bals_solve<N, true, kMany> : k_bals_solve<N, true, kDenseFew>)
+                 : (many ? k_bals_solve<N, false, kMany> : k_bals_solve<N, false, kDenseFew>);
   PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<ninst, kDenseThreads, smem, st>>>(n, degp1, szt, tailidx, mat, rhs, sol, Q, R, flags, work, stage, blocked);
   PHC_CHECK_LAUNCH();

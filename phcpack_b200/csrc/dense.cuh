@@ -156,6 +156,31 @@ __device__ __forceinline__ typename N::T group_sum(typename N::T a, int lanes) {
   return lanes == 8 ? N::add(a, md::shfl_xor(a, 4)) : a;
 }
 
+// sum += (conj) a_l b_l over l = l0, l0 + step, ... < n with a at stride lda
+// and b at stride ldb (numbers); the next pair is loaded before the products
+// of the present one (rows of A and Q come from L2 or memory, 300 to 1000
+// cycles away).  CONJ: conj(a); NEG: -a.
+template <class N, bool CONJ, bool NEG>
+__device__ __forceinline__ void dot_acc(md::msum<N> &sum, const double *a, long lda, const double *b, long ldb, int l0,
+                                        int step, int n) {
+  typedef typename N::T T;
+  if (l0 >= n) return;
+  T x = ldn_at<N>(a, (long)l0 * lda), y = ldn_at<N>(b, (long)l0 * ldb);
+#pragma unroll 1
+  for (int l = l0; l < n; l += step) {
+    const int nl = l + step < n ? l + step : l;
+    const T xn = ldn_at<N>(a, (long)nl * lda), yn = ldn_at<N>(b, (long)nl * ldb);
+    if (CONJ)
+      sum.cfma(x, y);
+    else if (NEG)
+      sum.fnma(x, y);
+    else
+      sum.fma(x, y);
+    x = xn;
+    y = yn;
+  }
+}
+
 // ------------------------------------------------------------- Householder
 // One column of a panel: the reflector of x = R[c.., c], m = n - c entries,
 // in PHCpack's convention (Matrices/dbl2_factorizations.cpp:374 real, :436
@@ -212,7 +237,7 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
     R beta = RN::zero();
     T inv = N::one();
     if (!md::is_zero(sigma)) {
-      T v0;
+      T v0 = N::zero();
       if constexpr (N::is_complex) {
         const R sq0 = N::norm2(x0);
         const R rad0 = RN::tr::sqrt(sq0);
@@ -227,17 +252,14 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
         const R mu = RN::tr::sqrt(RN::add(RN::mul(x0, x0), sigma));
         const bool cancel = !(md::lead(x0) <= 0.0);  // x0 - mu would cancel
         const R a = cancel ? RN::add(x0, mu) : RN::sub(x0, mu);
-        if (cancel) {
-          if (do_inv) inv = RN::neg(RN::tr::div(a, sigma));
-          v0 = do_beta ? RN::neg(RN::tr::div(sigma, a)) : a;
-        } else {
-          if (do_inv) inv = RN::tr::div(RN::one(), a);
-          v0 = a;
-        }
+        // sigma + v0^2 = -2 mu v0, so that beta = -v0 / mu: one division
+        // beside the other warp's, none of them waiting for another
+        if (do_inv) inv = cancel ? RN::neg(RN::tr::div(a, sigma)) : RN::tr::div(RN::one(), a);
+        if (do_beta) beta = cancel ? RN::tr::div(sigma, RN::mul(a, mu)) : RN::neg(RN::tr::div(a, mu));
       }
-      const R v0sq = N::norm2(v0);
-      if (do_beta) beta = md::mul_d(RN::tr::div(v0sq, RN::add(sigma, v0sq)), 2.0);
       if constexpr (N::is_complex) {
+        const R v0sq = N::norm2(v0);
+        if (do_beta) beta = md::mul_d(RN::tr::div(v0sq, RN::add(sigma, v0sq)), 2.0);
         if (do_inv) inv = N::mkc(RN::tr::div(v0.re, v0sq), RN::neg(RN::tr::div(v0.im, v0sq)));
       }
     }
@@ -509,7 +531,7 @@ __device__ void block_tiled_backsub(int dim, int szt, const double *U, int ldu, 
       md::msum<N> sum;
       sum.zero();
       if (i < szt)
-        for (int j = part; j < szt; j += 4) sum.fma(ldn_at<N>(inv, (long)i * szt + j), ldn_at<N>(b, off + j));
+        dot_acc<N, false, false>(sum, inv + (long)i * szt * N::width, 1, b + off * N::width, 1, part, 4, szt);
       const T acc = group4_sum<N>(sum.value());
       if (i < szt && part == 0) stn_at<N>(x, off + i, acc);
     }
@@ -519,7 +541,7 @@ __device__ void block_tiled_backsub(int dim, int szt, const double *U, int ldu, 
       md::msum<N> sum;
       sum.zero();
       if (r < off)
-        for (int j = part; j < szt; j += 4) sum.fma(ldn_at<N>(U, (long)r * ldu + off + j), ldn_at<N>(x, off + j));
+        dot_acc<N, false, false>(sum, U + ((long)r * ldu + off) * N::width, 1, x + off * N::width, 1, part, 4, szt);
       const T acc = group4_sum<N>(sum.value());
       if (r < off && part == 0) stn_at<N>(b, r, N::sub(ldn_at<N>(b, r), acc));
     }
@@ -538,7 +560,7 @@ __device__ void block_qhb(int n, const double *Q, const double *b, double *w) {
     md::msum<N> sum;
     sum.zero();
     if (i < n)
-      for (int j = part; j < n; j += 4) sum.cfma(ldn_at<N>(Q, (long)j * n + i), ldn_at<N>(b, j));
+      dot_acc<N, true, false>(sum, Q + (long)i * N::width, n, b, 1, part, 4, n);
     const T acc = group4_sum<N>(sum.value());
     if (i < n && part == 0) stn_at<N>(w, i, acc);
   }
@@ -547,58 +569,77 @@ __device__ void block_qhb(int n, const double *Q, const double *b, double *w) {
 
 // b_j -= A_{j-i+1} x for j = i..degp1-1 (Newton/dbl2_tail_kernels.cu:19
 // dbl2_bals_tail, all right hand sides of one stage at once), over the rows
-// of the stacked matrices A_1 .. A_{degp1-i}.  Quad-double: a thread per row
-// (its 450 FP64 cycles per product cover the uncoalesced loads), two or four
-// when the rows would leave threads idle.  Double and
-// double-double: four lanes per row, so that a load instruction touches 8
-// lines instead of 32 (a thread per row was bound by the L1 cache's
-// wavefronts) and a stage's rows fill the CTA.
+// of the stacked matrices A_1 .. A_{degp1-i}, which are contiguous.
+// Quad-double: a thread per row (its 450 FP64 cycles per product cover the
+// uncoalesced loads), two or four when the rows would leave threads idle.
+// Double and double-double: G lanes per row, so that a load instruction
+// touches few lines (a thread per row was bound by the L1 cache's
+// wavefronts), R rows to a group of lanes at a time with the next entries
+// loaded ahead, so that the loads of a stage, from L2 or memory, overlap.
+// Real double-double, dimension 64, degree 31: 4.87 ms with one row, 3.35
+// with two; complex double-double lost 4 % with two.
+template <class N>
+struct tail_shape {
+  static const int G = (N::tr::limbs == 1 && !N::is_complex) ? 8 : 4;
+  static const int R = N::tr::limbs == 1 ? (N::is_complex ? 2 : 4) : (N::is_complex ? 1 : 2);
+};
 template <class N>
 __device__ void block_tail_update(int n, int degp1, int i, const double *mat, double *rhs, const double *x) {
   typedef typename N::T T;
   const long nn = (long)n * n;
   const int rows = (degp1 - i) * n;
+  const double *A = mat + nn * N::width;       // row r of A_1, A_2, ...
+  double *b = rhs + (long)i * n * N::width;    // its entry of b_i, b_{i+1}, ...
   if constexpr (N::tr::limbs > 2) {
     const int G = rows * 4 <= (int)blockDim.x ? 4 : (rows * 2 <= (int)blockDim.x ? 2 : 1);
     const int grp = threadIdx.x / G, part = threadIdx.x % G, ngrp = blockDim.x / G;
     for (int base = 0; base < rows; base += ngrp) {
       const int r = base + grp;
-      const double *A = mat + (nn + (long)r * n) * N::width;
-      double *bj = rhs + ((long)i * n + r) * N::width;
       md::msum<N> sum;
       sum.zero();
       if (r < rows) {
-        if (part == 0) {
-          T v;
-          md::ldn(bj, v);
-          sum.set(v);
-        }
-        for (int l = part; l < n; l += G) sum.fnma(ldn_at<N>(A, l), ldn_at<N>(x, l));
+        if (part == 0) sum.set(ldn_at<N>(b, r));
+        dot_acc<N, false, true>(sum, A + (long)r * n * N::width, 1, x, 1, part, G, n);
       }
       T v = sum.value();
       if (G > 1) v = N::add(v, md::shfl_xor(v, 1));
       if (G > 2) v = N::add(v, md::shfl_xor(v, 2));
-      if (r < rows && part == 0) md::stn(bj, v);
+      if (r < rows && part == 0) stn_at<N>(b, r, v);
     }
   } else {
-    const int grp = threadIdx.x >> 2, part = threadIdx.x & 3, ngrp = blockDim.x >> 2;
-    for (int base = 0; base < rows; base += ngrp) {
-      const int r = base + grp;
-      // the stacked matrices are contiguous: row r of A_1, A_2, ...
-      const double *A = mat + (nn + (long)r * n) * N::width;
-      double *bj = rhs + ((long)i * n + r) * N::width;
-      md::msum<N> sum;
-      sum.zero();
-      if (r < rows) {
-        if (part == 0) {
-          T v;
-          md::ldn(bj, v);
-          sum.set(v);
-        }
-        for (int l = part; l < n; l += 4) sum.fnma(ldn_at<N>(A, l), ldn_at<N>(x, l));
+    const int G = tail_shape<N>::G, R = tail_shape<N>::R;
+    const int grp = threadIdx.x / G, part = threadIdx.x % G, ngrp = blockDim.x / G;
+    for (int base = 0; base < rows; base += R * ngrp) {
+      md::msum<N> sum[R];
+      const double *a[R];
+      T e[R];
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int r = base + u * ngrp + grp;
+        sum[u].zero();
+        a[u] = A + (long)(r < rows ? r : 0) * n * N::width;
+        e[u] = part < n ? ldn_at<N>(a[u], part) : N::zero();
+        if (part == 0 && r < rows) sum[u].set(ldn_at<N>(b, r));
       }
-      const T v = group4_sum<N>(sum.value());
-      if (r < rows && part == 0) md::stn(bj, v);
+#pragma unroll 1
+      for (int l = part; l < n; l += G) {
+        const int nl = l + G < n ? l + G : l;
+        const T xl = ldn_at<N>(x, l);
+        T next[R];
+#pragma unroll
+        for (int u = 0; u < R; ++u) next[u] = ldn_at<N>(a[u], nl);
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          sum[u].fnma(e[u], xl);
+          e[u] = next[u];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int r = base + u * ngrp + grp;
+        const T v = group_sum<N>(sum[u].value(), G);
+        if (part == 0 && r < rows) stn_at<N>(b, r, v);
+      }
     }
   }
   __syncthreads();
