@@ -24,6 +24,7 @@ namespace phc {
 
 static const int kMaxWarpsPerBlock = 8;
 static const int kMaxSmem = 227 * 1024;
+static const int kSquareDims = 256;  // variables whose squares may be kept
 // Polynomials up to which a CTA takes one: 8 warps each, so that one wave of
 // CTAs still gives every SM 8 polynomials.  One system of 8 polynomials of 12
 // monomials (degree 15, complex double-double): 68 us shared, 332 with a warp
@@ -41,12 +42,42 @@ __device__ __forceinline__ void stage_inputs(const double *__restrict__ xin, dou
   }
 }
 
+// The squares of the variables that have an exponent above 2 in the monomials
+// m0..m1-1, into sq (dim series): a product each, one less wherever they
+// occur.  X in shared memory.  Called by the whole CTA; the caller
+// synchronises before they are read.
+template <class N, bool BIG>
+__device__ const double *needed_squares(int dim, int deg, int maxvar, int m0, int m1, const int *__restrict__ nvr,
+                                        const int *__restrict__ idx, const int *__restrict__ exps, const double *X,
+                                        double *sq) {
+  __shared__ unsigned need[kSquareDims / 32];
+  if (threadIdx.x < kSquareDims / 32) need[threadIdx.x] = 0u;
+  __syncthreads();
+  for (int m = m0 + threadIdx.x; m < m1; m += blockDim.x) {
+    const int k = nvr[m];
+    if (k < 1 || k > maxvar) continue;
+    for (int v = 0; v < k; ++v) {
+      const int i = idx[(long)m * maxvar + v];
+      if (i >= 0 && i < dim && exps[(long)m * maxvar + v] > 2) atomicOr(&need[i >> 5], 1u << (i & 31));
+    }
+  }
+  __syncthreads();
+  const int S = (deg + 1) * N::width;
+  const typename wser<N, BIG>::map map(deg, threadIdx.x & 31, 0);
+  for (int i = threadIdx.x >> 5; i < dim; i += blockDim.x >> 5) {
+    if (!((need[i >> 5] >> (i & 31)) & 1u)) continue;
+    const typename N::T z = wser<N, BIG>::conv(X + i * S, X + i * S, map);
+    if (map.valid) md::stn(sq + i * S + map.kout() * N::width, z);
+  }
+  return sq;
+}
+
 // A warp per polynomial.  BIG (degrees 32..191): one more scratch series per
 // warp (the value); the inputs are staged in shared memory when they fit
 // beside the scratch and read from global memory otherwise.
 template <class N, bool BIG>
 __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, N::width <= 4 ? 2 : 1)
-    k_system_evaldiff(int dim, int deg, int maxvar, int wpb, int stage, const int *__restrict__ mon_off,
+    k_system_evaldiff(int dim, int deg, int maxvar, int wpb, int stage, int squares, const int *__restrict__ mon_off,
                       const int *__restrict__ nvr, const int *__restrict__ idx, const int *__restrict__ exps,
                       const double *__restrict__ cst, const double *__restrict__ cff,
                       const double *__restrict__ input, double *__restrict__ output) {
@@ -62,20 +93,26 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, N::width <= 4 ? 2 : 1)
     X = sm;
     scr = sm + ((dim * S + 1) & ~1);
   }
-  __syncthreads();
   const int warp = threadIdx.x >> 5;
   const int p = p0 + warp;
+  const long sp = (long)s * dim + p;
+  const double *X2 = nullptr;
+  if (squares) {
+    X2 = needed_squares<N, BIG>(dim, deg, maxvar, mon_off[(long)s * dim + p0], mon_off[(long)s * dim + min(p0 + wpb, dim)],
+                                nvr, idx, exps, X, scr);
+    scr += (dim * S + 1) & ~1;
+  }
+  __syncthreads();
   if (p >= dim) return;
   scr += (long)warp * (warp_slots(maxvar) + (BIG ? 1 : 0)) * S;
-  const long sp = (long)s * dim + p;
-  warp_poly_evaldiff<N, BIG>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, cst + sp * S, cff, X,
+  warp_poly_evaldiff<N, BIG>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, cst + sp * S, cff, X, X2,
                              scr, output + sp * (dim + 1) * S);
 }
 
 // A CTA per polynomial, its monomials shared by the warps.
 template <class N, bool BIG>
 __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, N::width <= 4 ? 2 : 1)
-    k_poly_evaldiff(int dim, int deg, int maxvar, int stage, const int *__restrict__ mon_off,
+    k_poly_evaldiff(int dim, int deg, int maxvar, int stage, int squares, const int *__restrict__ mon_off,
                     const int *__restrict__ nvr, const int *__restrict__ idx, const int *__restrict__ exps,
                     const double *__restrict__ cst, const double *__restrict__ cff, const double *__restrict__ input,
                     double *__restrict__ output) {
@@ -90,8 +127,13 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, N::width <= 4 ? 2 : 1)
     X = scr;
     scr += (dim * S + 1) & ~1;
   }
+  const double *X2 = nullptr;
+  if (squares) {
+    X2 = needed_squares<N, BIG>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, X, scr);
+    scr += (dim * S + 1) & ~1;
+  }
   __syncthreads();
-  cta_poly_evaldiff<N, BIG>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, cst + sp * S, cff, X,
+  cta_poly_evaldiff<N, BIG>(dim, deg, maxvar, mon_off[sp], mon_off[sp + 1], nvr, idx, exps, cst + sp * S, cff, X, X2,
                             scr, rows, output + sp * (dim + 1) * S);
 }
 
@@ -104,6 +146,13 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
   const long series = (long)S * sizeof(double);
   const long xs = (long)((dim * S + 1) & ~1) * sizeof(double);
   const int tuned = tune_get(kTuneEvalWarps);  // warps per CTA chosen by the autotuner
+  // The squares of the variables beside the inputs, for short series, while
+  // two CTAs of the built-in shape still share an SM (1024 systems n = 32
+  // with exponents up to 3: one in nine products saved, 24.2 -> 22.2 ms;
+  // exponents up to 2: 20.2 -> 20.5).  Decided by the sizes alone, so that
+  // every arrangement forms the same products.
+  const long warp8 = (dim < kMaxWarpsPerBlock ? dim : kMaxWarpsPerBlock) * (long)warp_slots(maxvar) * series;
+  const int squares = !big && dim <= kSquareDims && warp8 + 2 * xs + 1024 <= 114 * 1024;
   // A warp per polynomial leaves most of the GPU idle on a few systems, and
   // each warp's products follow one another.  While the polynomials are
   // fewer than kSplitPolys a CTA takes one polynomial and shares its
@@ -112,15 +161,16 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
     const long per_warp = (warp_slots(maxvar) + maxvar + 1) * series;
     const long rows = (long)(((dim + 1) * S + 1) & ~1) * sizeof(double);
     int nw = kMaxWarpsPerBlock;
-    while (nw > 2 && rows + nw * per_warp > kMaxSmem - 1024) --nw;
-    long smem = rows + nw * per_warp;
+    const long fixed = rows + (squares ? 2 * xs : 0);
+    while (nw > 2 && fixed + nw * per_warp > kMaxSmem - 1024) --nw;
+    long smem = fixed + nw * per_warp;
     if (smem <= kMaxSmem - 1024) {
-      const int stage = smem + xs <= 200 * 1024;
-      if (stage) smem += xs;
+      const int stage = squares || smem + xs <= 200 * 1024;
+      if (stage && !squares) smem += xs;
       auto kern = big ? k_poly_evaldiff<N, true> : k_poly_evaldiff<N, false>;
       PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      kern<<<(unsigned)(nsys * dim), nw * 32, smem, stream>>>(dim, deg, maxvar, stage, mon_off, nvr, idx, exps, cst,
-                                                               cff, input, output);
+      kern<<<(unsigned)(nsys * dim), nw * 32, smem, stream>>>(dim, deg, maxvar, stage, squares, mon_off, nvr, idx, exps,
+                                                               cst, cff, input, output);
       PHC_CHECK_LAUNCH();
       return PHC_OK;
     }
@@ -135,7 +185,7 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
   while (wpb > 1 && (long)wpb * per_warp > kMaxSmem) --wpb;
   const long scr = (long)wpb * per_warp;
   int stage = (scr + xs) <= 200 * 1024;
-  const long smem = scr + (stage ? xs : 0);
+  const long smem = scr + (stage ? xs : 0) + (squares ? xs : 0);
   if (smem > kMaxSmem) {
     set_error("system_evaldiff: %ld bytes of shared memory needed (maxvar %d, degree %d)", smem, maxvar, deg);
     return PHC_ERR_LIMIT;
@@ -144,7 +194,7 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
   PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int bps = (dim + wpb - 1) / wpb;
   const long grid = (long)nsys * bps;
-  kern<<<(unsigned)grid, wpb * 32, smem, stream>>>(dim, deg, maxvar, wpb, stage, mon_off, nvr, idx, exps, cst, cff,
+  kern<<<(unsigned)grid, wpb * 32, smem, stream>>>(dim, deg, maxvar, wpb, stage, squares, mon_off, nvr, idx, exps, cst, cff,
                                                    input, output);
   PHC_CHECK_LAUNCH();
   return PHC_OK;

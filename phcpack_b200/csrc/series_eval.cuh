@@ -134,9 +134,10 @@ struct wser {
 };
 
 // Shared-memory series slots a warp needs for monomials of up to maxvar
-// variables: the coefficient, a temporary, f_0..f_{k-2}, b_0..b_{k-3}.
+// variables: the coefficient and a temporary (which takes b_0 after the
+// common factors), f_0..f_{k-2}, b_1..b_{k-3}.
 __host__ __device__ inline int warp_slots(int maxvar) {
-  int s = 2 * maxvar - 1;
+  int s = 2 * maxvar - 2;
   return s < 3 ? 3 : s;
 }
 
@@ -157,7 +158,8 @@ __host__ __device__ inline int warp_slots(int maxvar) {
 // across it, which the product needs for independent operations in flight
 // (FP64 latency, not the pipe, limited the evaluation), and a copy per kind
 // of product would not fit the instruction cache.
-// X: dim series (shared memory or global); scr: warp_slots(maxvar) series of
+// X: dim series (shared memory or global); X2: their squares where a monomial
+// has an exponent above 2 (a factor x^2 is then one product), or null; scr: warp_slots(maxvar) series of
 // shared memory.  A malformed monomial (variable count, index or exponent
 // out of range) is skipped rather than read out of bounds; the host entry
 // points reject such supports before any launch.  Returns the number of
@@ -165,15 +167,15 @@ __host__ __device__ inline int warp_slots(int maxvar) {
 template <class N, bool BIG, class Sink>
 __device__ __forceinline__ int warp_monomial(const wser<N, BIG> &ws, int dim, int maxvar, int k,
                                              const int *__restrict__ ix, const int *__restrict__ ex,
-                                             const double *__restrict__ cffm, const double *X, double *scr,
-                                             Sink &sink) {
+                                             const double *__restrict__ cffm, const double *X, const double *X2,
+                                             double *scr, Sink &sink) {
   typedef typename N::T T;
   const int S = ws.n1 * N::width;
   bool ok = (k >= 1 && k <= maxvar);
   for (int v = 0; ok && v < k; ++v) ok = (ix[v] >= 0 && ix[v] < dim && ex[v] >= 1);
   if (!ok) return 0;
   double *const F = scr + 2 * S;                 // f_0 .. f_{k-2}
-  double *const B = scr + (1 + maxvar) * S;      // b_0 .. b_{k-3}
+  double *const B = scr + maxvar * S;            // b_1 .. b_{k-3} (B + i S)
   ws.copy(cffm, scr);
   __syncwarp();
   int cslot = 0;         // c is scratch series 0 or 1
@@ -183,6 +185,7 @@ __device__ __forceinline__ int warp_monomial(const wser<N, BIG> &ws, int dim, in
 #pragma unroll 1
   for (;;) {
     const double *C = scr + cslot * S;
+    double *const b0 = scr + (cslot ^ 1) * S;
     const double *x, *y;
     double *dst = nullptr;  // scratch series that takes the product
     int var = -1;           // variable whose derivative it is
@@ -192,11 +195,12 @@ __device__ __forceinline__ int warp_monomial(const wser<N, BIG> &ws, int dim, in
       r = 1;
     }
     if (v < k) {
-      x = X + ix[v] * S;
+      const bool two = X2 != nullptr && r + 1 < ex[v];
+      x = (two ? X2 : X) + ix[v] * S;
       y = C;
       cslot ^= 1;
       dst = scr + cslot * S;
-      ++r;
+      r += two ? 2 : 1;
     } else if (j < nprod) {
       if (j < k - 1) {
         x = j == 0 ? C : F + (j - 1) * S;
@@ -209,17 +213,17 @@ __device__ __forceinline__ int warp_monomial(const wser<N, BIG> &ws, int dim, in
         value = true;
       } else if (j < 2 * k - 2) {
         const int i = j - k;
-        x = i == 0 ? X + ix[k - 1] * S : B + (i - 1) * S;
+        x = i == 0 ? X + ix[k - 1] * S : (i == 1 ? b0 : B + (i - 1) * S);
         y = X + ix[k - 2 - i] * S;
-        dst = B + i * S;
+        dst = i == 0 ? b0 : B + i * S;
       } else if (j == 2 * k - 2) {
-        x = k == 2 ? X + ix[0] * S : B + (k - 3) * S;
+        x = k == 2 ? X + ix[0] * S : (k == 3 ? b0 : B + (k - 3) * S);
         y = C;
         var = k == 2 ? 1 : 0;
       } else {
         const int i = j - (2 * k - 1);
         x = F + i * S;
-        y = i == k - 3 ? X + ix[k - 1] * S : B + (k - 4 - i) * S;
+        y = i == k - 3 ? X + ix[k - 1] * S : (i == k - 4 ? b0 : B + (k - 4 - i) * S);
         var = i + 1;
       }
       ++j;
@@ -334,14 +338,14 @@ template <class N, bool BIG>
 __device__ __forceinline__ void warp_poly_evaldiff(int dim, int deg, int maxvar, int m0, int m1,
                                                    const int *__restrict__ nvr, const int *__restrict__ idx,
                                                    const int *__restrict__ exps, const double *__restrict__ cst,
-                                                   const double *__restrict__ cff, const double *X, double *scr,
-                                                   double *out) {
+                                                   const double *__restrict__ cff, const double *X,
+                                                   const double *X2, double *scr, double *out) {
   const wser<N, BIG> ws(deg, threadIdx.x & 31);
   const long S = (long)ws.n1 * N::width;
   row_sink<N, BIG> sink(ws, out, scr + warp_slots(maxvar) * S, dim, cst);
   for (int mon = m0; mon < m1; ++mon)
     warp_monomial<N, BIG>(ws, dim, maxvar, nvr[mon], idx + (long)mon * maxvar, exps + (long)mon * maxvar,
-                          cff + mon * S, X, scr, sink);
+                          cff + mon * S, X, X2, scr, sink);
   sink.finish(dim);
 }
 
@@ -372,8 +376,8 @@ template <class N, bool BIG>
 __device__ __forceinline__ void cta_poly_evaldiff(int dim, int deg, int maxvar, int m0, int m1,
                                                   const int *__restrict__ nvr, const int *__restrict__ idx,
                                                   const int *__restrict__ exps, const double *__restrict__ cst,
-                                                  const double *__restrict__ cff, const double *X, double *scr,
-                                                  double *rows, double *out) {
+                                                  const double *__restrict__ cff, const double *X,
+                                                  const double *X2, double *scr, double *rows, double *out) {
   typedef typename N::T T;
   const int W = N::width;
   const wser<N, BIG> ws(deg, threadIdx.x & 31);
@@ -393,7 +397,7 @@ __device__ __forceinline__ void cta_poly_evaldiff(int dim, int deg, int maxvar, 
     if (mon < m1) {
       slot_sink<N, BIG> sink(ws, mine + warp_slots(maxvar) * S);
       k = warp_monomial<N, BIG>(ws, dim, maxvar, nvr[mon], idx + (long)mon * maxvar, exps + (long)mon * maxvar,
-                                cff + (long)mon * S, X, mine, sink);
+                                cff + (long)mon * S, X, X2, mine, sink);
     }
     if ((threadIdx.x & 31) == 0) kdone[warp] = k;
     __syncthreads();

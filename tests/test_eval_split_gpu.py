@@ -41,3 +41,16 @@ def test_shared_monomials_match_oracle(prec, cplx, nsys, dim, deg, nmon, maxvar)
     scale = ORC.system_evaldiff(abs_batch(b))
     for knob in (0, 4):  # shared; four polynomials per CTA
         assert check_scaled(evaluate(b, knob), ref, scale, prec, cplx, RTOL[prec]) <= 1.0
+
+
+@pytest.mark.parametrize("prec,cplx,dim,deg,expmax", [(1, False, 3, 5, 6), (2, True, 9, 31, 5), (2, False, 5, 31, 3),
+                                                      (4, False, 4, 9, 4), (2, True, 40, 2, 4)])
+def test_squares_match_oracle(prec, cplx, dim, deg, expmax):
+    # a warp per polynomial with the squares of the variables at hand:
+    # exponents 3, 4, 5, ... are one, one and a half, two squares ..., and a
+    # last group of polynomials smaller than the CTA
+    b = wl.eval_batch(400 + dim, 1, dim, deg, 5, 3, prec, cplx, expmax=expmax)
+    ref = ORC.system_evaldiff(b)
+    scale = ORC.system_evaldiff(abs_batch(b))
+    for knob in (2, 8):
+        assert check_scaled(evaluate(b, knob), ref, scale, prec, cplx, RTOL[prec]) <= 1.0
