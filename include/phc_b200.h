@@ -41,8 +41,9 @@ int phc_abi_version(void);
  *           batch of at most 1184 polynomials takes a CTA per polynomial
  *           instead, its monomials shared by the warps);
  *   knob 1: variant of the split tracker's kernel, 1 the 64-register one
- *           (8 paths per SM), 2 the 72-register one (7 paths per SM) (the
- *           rule: 2 when the batch fits in one wave at 7 per SM);
+ *           (8 paths per SM), 2 the 72-register one (7 paths per SM; the
+ *           128-register one when the batch or knob 2 asks for no more than
+ *           4) (the rule: 2 when the batch fits in one wave at 7 per SM);
  *   knob 2: paths the tracker runs at once per SM, 1..32, at most what the
  *           occupancy allows (the rule: that maximum); the work queue hands
  *           out the other paths as paths finish;

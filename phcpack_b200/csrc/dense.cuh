@@ -6,9 +6,9 @@
 // One CTA owns one instance.  Matrices are row-major, limb-interleaved, in
 // global memory (one instance's Q, R and WY panels stay resident in L2);
 // shared memory holds the Householder vector, the reflector coefficients,
-// the current solution vector and the reduction buffers.  Norms and dot
-// products are warp-shuffle reductions followed by a shared-memory pass
-// across warps.
+// the current solution vector and the reduction buffers.  Dot products are
+// shared by groups of four or eight lanes; the norms of the skip rules are
+// formed by every warp for itself.
 #pragma once
 #include "md.cuh"
 #include "ozaki.cuh"

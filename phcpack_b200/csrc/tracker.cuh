@@ -563,8 +563,8 @@ __device__ __forceinline__ void column_update(int n, double *X, int c, const dou
 // reciprocals dinv[k] = 1 / u_kk are kept for the back substitution (NaN
 // for a zero pivot).  One warp alone, no CTA barrier (the other warps of the
 // CTA stay free).  Per column: lane i (k <= i < n) holds a_ik and forms its
-// reciprocal while the warp finds the largest candidate (warp_max_nonneg
-// and one ballot), so that 1 / a_kk is a shuffle away once the pivot row is
+// reciprocal while the warp finds the largest candidate (a reduction of the
+// high words and a ballot; the low words when two rows tie), so that 1 / a_kk is a shuffle away once the pivot row is
 // known, and stores its multiplier.  The trailing update gives every column
 // j > k to 32 / (n-k-1) lanes that share its rows: each has read the two
 // entries of the swap before anything is written, so the swap costs no pass

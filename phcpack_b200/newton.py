@@ -30,10 +30,10 @@ class DeviceNewton:
     """A batch of systems resident on the device for repeated Newton solves at
     a fixed working degree: each step is phc_newton_step (evaluate and
     differentiate, linearise, block-Toeplitz least squares, update; four
-    launches and a memset, all on one stream, no host synchronisation), and
-    the steps of one solve, from the start series on, can be captured once in
-    a CUDA graph and replayed: one graph launch per solve instead of five
-    launches per step.  The start series and the skip-rule flags (zeroQ = 1,
+    launches, all on one stream, no host synchronisation), and the steps of
+    one solve, from the start series on, can be captured once in a CUDA graph
+    and replayed: one graph launch per solve instead of four launches per
+    step.  The start series and the skip-rule flags (zeroQ = 1,
     noqr = 0, tail index 1, as phc_newton_host starts them) are restored on
     the device at the start of every solve."""
 
