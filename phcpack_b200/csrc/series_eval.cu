@@ -29,7 +29,11 @@ static const int kSquareDims = 256;  // variables whose squares may be kept
 // CTAs still gives every SM 8 polynomials.  One system of 8 polynomials of 12
 // monomials (degree 15, complex double-double): 68 us shared, 332 with a warp
 // per polynomial; 512 polynomials at degree 95: 1.04 ms against 2.7.
-static const long kSplitPolys = 148 * 8;
+// A monomial of one variable is one product (in double also two variables
+// are little work): there the CTA's staging and summing outweigh the shared
+// products beyond two CTAs per SM (960 polynomials of 6 one-variable
+// monomials in double: 35 us shared, 33 with a warp per polynomial).
+static const long kSplitPolys = 148 * 8, kSplitPolysShort = 148 * 2;
 
 // Input series of a system, n doubles, into shared memory.
 __device__ __forceinline__ void stage_inputs(const double *__restrict__ xin, double *Xs, int n) {
@@ -157,7 +161,8 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
   // each warp's products follow one another.  While the polynomials are
   // fewer than kSplitPolys a CTA takes one polynomial and shares its
   // monomials among its warps, when the rows fit in shared memory.
-  if (tuned == 0 && (long)nsys * dim <= kSplitPolys) {
+  const bool short_work = maxvar == 1 || (maxvar == 2 && N::tr::limbs == 1);
+  if (tuned == 0 && (long)nsys * dim <= (short_work ? kSplitPolysShort : kSplitPolys)) {
     const long per_warp = (warp_slots(maxvar) + maxvar + 1) * series;
     const long rows = (long)(((dim + 1) * S + 1) & ~1) * sizeof(double);
     int nw = kMaxWarpsPerBlock;
