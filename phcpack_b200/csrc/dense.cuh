@@ -195,10 +195,54 @@ __device__ __forceinline__ void dot_acc(md::msum<N> &sum, const double *a, long 
 // conj(R_cj) + (1/v0) D_j, D_j = sum_{i>c} conj(R_ij) x_i, and D_c is sigma
 // itself: the first sweep needs nothing of the chain and also replaces the
 // norm's reduction, and the warps 0 and 1 form beta and 1/v0 side by side.
-// Four barriers per column.  Entry (i, j) of R sits at Rm[(i - r0) * ld +
-// (j - c0)]: the whole matrix (r0 = c0 = 0, ld = ncols) or a panel of it
-// staged in shared memory.  Leaves v in S.v (m numbers) and beta in
-// S.misc[0] (a real number).
+// Four barriers per column.
+//
+// Everything is formed with the column scaled by 2^-E, the power of two above
+// the largest x_i below the diagonal (exact, no other bits away from the ends
+// of the range): unscaled, sigma and the D_j lose their lower limbs, and 1/v0
+// overflows, where small x_i stand below an x0 of order one.  A column is
+// left alone (beta = 0) where the reference's beta is zero: when the squares
+// of all x_i underflow, or the square of v0 does.
+//
+// Entry (i, j) of R sits at Rm[(i - r0) * ld + (j - c0)]: the whole matrix
+// (r0 = c0 = 0, ld = ncols) or a panel of it staged in shared memory.  Leaves
+// v in S.v (m numbers) and beta in S.misc[0] (a real number).
+static const int kReflectUnder = -537;  // the square of a number below 2^-537 underflows
+
+// High word of the larger of |re| and |im| of number i at p: orders numbers by
+// size, a NaN above all.
+template <class N>
+__device__ __forceinline__ unsigned lead_word(const double *p, long i) {
+  p += i * N::width;
+  const unsigned a = (unsigned)__double2hiint(p[0]) & 0x7fffffffu;
+  return N::is_complex ? max(a, (unsigned)__double2hiint(p[N::tr::limbs]) & 0x7fffffffu) : a;
+}
+// Exponent E of the scale of a column, mx and x0 the high words of its largest
+// entry below the diagonal and of the diagonal one: the entries are below 2^E,
+// and E is not so far below x0's that x0's square would overflow.
+__device__ __forceinline__ int reflect_exponent(unsigned mx, unsigned x0) {
+  if (mx == 0u) return 0;
+  return max(min((int)(mx >> 20) - 1022, 1000), max((int)(x0 >> 20) - 1322, -1000));
+}
+__device__ __forceinline__ double pow2(int e) {  // 0 when it would not be a normal number
+  return e < -1022 ? 0.0 : __hiloint2double((1023 + e) << 20, 0);
+}
+// every limb times a power of two
+__device__ __forceinline__ double mul_pow2(double a, double s) { return __dmul_rn(a, s); }
+__device__ __forceinline__ md::dd mul_pow2(const md::dd &a, double s) {
+  return md::mk(__dmul_rn(a.hi, s), __dmul_rn(a.lo, s));
+}
+__device__ __forceinline__ md::qd mul_pow2(const md::qd &a, double s) {
+  return md::mkq(__dmul_rn(a.x[0], s), __dmul_rn(a.x[1], s), __dmul_rn(a.x[2], s), __dmul_rn(a.x[3], s));
+}
+template <class R>
+__device__ __forceinline__ md::cx<R> mul_pow2(const md::cx<R> &a, double s) {
+  md::cx<R> r;
+  r.re = mul_pow2(a.re, s);
+  r.im = mul_pow2(a.im, s);
+  return r;
+}
+
 template <class N>
 __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_smem &S, int r0, int c0) {
   typedef typename N::T T;
@@ -206,6 +250,11 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
   typedef md::num<R, false> RN;
   const int m = n - c, nc = e - c;
   double *col = Rm + ((long)(c - r0) * ld + (c - c0)) * N::width;  // entry (c, c)
+  // the scale, by every warp for itself
+  unsigned mx = 0u;
+  for (int i = 1 + (threadIdx.x & 31); i < m; i += 32) mx = max(mx, lead_word<N>(col, (long)i * ld));
+  const int E = reflect_exponent(__reduce_max_sync(0xffffffffu, mx), lead_word<N>(col, 0));
+  const double down = pow2(-E);
   {
     // D_j for the panel's columns, 4 lanes per column (8 when the columns
     // are few and long)
@@ -216,7 +265,10 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
       md::msum<N> sum;
       sum.zero();
       if (j < nc)
-        for (int i = 1 + part; i < m; i += G) sum.cfma(ldn_at<N>(col, (long)i * ld + j), ldn_at<N>(col, (long)i * ld));
+        for (int i = 1 + part; i < m; i += G) {
+          const T x = mul_pow2(ldn_at<N>(col, (long)i * ld), down);
+          sum.cfma(j == 0 ? x : ldn_at<N>(col, (long)i * ld + j), x);
+        }
       const T d = group_sum<N>(sum.value(), G);
       if (j < nc && part == 0) stn_at<N>(S.w, j, d);
     }
@@ -224,7 +276,7 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
   __syncthreads();
   const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   if (warp < 2) {
-    const T x0 = ldn_at<N>(col, 0);
+    const T x0 = mul_pow2(ldn_at<N>(col, 0), down);
     R sigma;
     {
       const T d0 = ldn_at<N>(S.w, 0);
@@ -236,7 +288,7 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
     const bool do_beta = warp == 0, do_inv = warp == 1 || nwarp == 1;
     R beta = RN::zero();
     T inv = N::one();
-    if (!md::is_zero(sigma)) {
+    if (!md::is_zero(sigma) && !(md::lead(sigma) < pow2(2 * (kReflectUnder - E)))) {
       T v0 = N::zero();
       if constexpr (N::is_complex) {
         const R sq0 = N::norm2(x0);
@@ -248,19 +300,19 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
           mu = RN::tr::div(mu, rad0);
           v0 = N::mkc(RN::sub(x0.re, RN::mul(mu, x0.re)), RN::sub(x0.im, RN::mul(mu, x0.im)));
         }
+        const R v0sq = N::norm2(v0);
+        const bool under = md::lead(v0sq) < pow2(2 * (kReflectUnder - E));
+        if (do_beta && !under) beta = md::mul_d(RN::tr::div(v0sq, RN::add(sigma, v0sq)), 2.0);
+        if (do_inv) inv = N::mkc(RN::tr::div(v0.re, v0sq), RN::neg(RN::tr::div(v0.im, v0sq)));
       } else {
         const R mu = RN::tr::sqrt(RN::add(RN::mul(x0, x0), sigma));
         const bool cancel = !(md::lead(x0) <= 0.0);  // x0 - mu would cancel
         const R a = cancel ? RN::add(x0, mu) : RN::sub(x0, mu);
+        const bool under = cancel && md::lead(sigma) < __dmul_rn(md::lead(a), pow2(kReflectUnder - E));
         // sigma + v0^2 = -2 mu v0, so that beta = -v0 / mu: one division
         // beside the other warp's, none of them waiting for another
         if (do_inv) inv = cancel ? RN::neg(RN::tr::div(a, sigma)) : RN::tr::div(RN::one(), a);
-        if (do_beta) beta = cancel ? RN::tr::div(sigma, RN::mul(a, mu)) : RN::neg(RN::tr::div(a, mu));
-      }
-      if constexpr (N::is_complex) {
-        const R v0sq = N::norm2(v0);
-        if (do_beta) beta = md::mul_d(RN::tr::div(v0sq, RN::add(sigma, v0sq)), 2.0);
-        if (do_inv) inv = N::mkc(RN::tr::div(v0.re, v0sq), RN::neg(RN::tr::div(v0.im, v0sq)));
+        if (do_beta && !under) beta = cancel ? RN::tr::div(sigma, RN::mul(a, mu)) : RN::neg(RN::tr::div(a, mu));
       }
     }
     if ((threadIdx.x & 31) == 0) {
@@ -279,12 +331,13 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
         T v = N::one();
         if (t > 0) {
           v = ldn_at<N>(col, (long)t * ld);
-          if (!trivial) v = N::mul(v, inv);
+          if (!trivial) v = N::mul(mul_pow2(v, down), inv);
         }
         stn_at<N>(S.v, t, v);
       } else if (!trivial) {
         const int j = t - m;
-        const T d = md::mul_add<N>(N::conj(ldn_at<N>(col, j)), inv, ldn_at<N>(S.w, j));
+        const T dj = ldn_at<N>(S.w, j);  // D_j 2^-E, at j = 0 sigma 4^-E
+        const T d = md::mul_add<N>(N::conj(ldn_at<N>(col, j)), inv, j == 0 ? mul_pow2(dj, pow2(E)) : dj);
         stn_at<N>(S.w, j, N::scale(d, beta));
       }
     }
