@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(kDenseThreads, PER_SM)
         active &= ~(1u << (src & 15));
       } else {
         active |= 1u << (src & 15);
-        block_tail_update<N>(n, blocked ? min(degp1, tail0 + (src | 3) + 1) : degp1, i, A, b, S.x);
+        const int je = blocked ? min(degp1, tail0 + (src | 3) + 1) : degp1;
+        block_tail_update<N>(n, (je - i) * n, A + nn * W, b + (long)i * n * W, S.x);
       }
       if constexpr (N::tr::limbs == 4 && !N::is_complex) {
         const int u = src + 1;
@@ -152,9 +153,19 @@ __global__ void __launch_bounds__(kDenseThreads, PER_SM)
           const int ns = (u & 15) == 0 ? 16 : ((u & 7) == 0 ? 8 : 4);
           const int j0 = tail0 + u, j1 = ns == 16 ? degp1 : min(degp1, j0 + ns);
           const unsigned mask = (active >> ((u - ns) & 15)) & ((1u << ns) - 1u);
-          if (j0 < j1 && mask)
-            block_tail_i8(n, A, b, x, tail0 - 1 + u - ns, ns, mask, j0, j1,
-                          reinterpret_cast<unsigned char *>(sm + dense_smem_doubles(n, szt, W)));
+          if (j0 < j1 && mask) {
+            const int s0 = tail0 - 1 + u - ns;
+            const int m = block_tail_i8(n, A, b, x, s0, ns, mask, j0, j1,
+                                        reinterpret_cast<unsigned char *>(sm + dense_smem_doubles(n, szt, W)));
+            // what is left, from A_m on, source by source
+            for (int s = s0; s < s0 + ns; ++s) {
+              const int j = max(j0, s + m);
+              if (j >= j1 || !((mask >> (s - s0)) & 1u)) continue;
+              for (int l = threadIdx.x; l < n; l += blockDim.x) stn_at<N>(S.w, l, ldn_at<N>(x, (long)s * n + l));
+              __syncthreads();
+              block_tail_update<N>(n, (j1 - j) * n, A + (j - s) * nn * W, b + (long)j * n * W, S.w);
+            }
+          }
         }
       }
       const double *bi = b + (long)i * n * W;

@@ -620,9 +620,10 @@ __device__ void block_qhb(int n, const double *Q, const double *b, double *w) {
   __syncthreads();
 }
 
-// b_j -= A_{j-i+1} x for j = i..degp1-1 (Newton/dbl2_tail_kernels.cu:19
-// dbl2_bals_tail, all right hand sides of one stage at once), over the rows
-// of the stacked matrices A_1 .. A_{degp1-i}, which are contiguous.
+// b -= A x over rows rows: those of the matrices A_k, A_{k+1}, ... and of the
+// right hand sides b_j, b_{j+1}, ..., stacked and contiguous
+// (Newton/dbl2_tail_kernels.cu:19 dbl2_bals_tail, the targets of one stage at
+// once).
 // Quad-double: a thread per row (its 450 FP64 cycles per product cover the
 // uncoalesced loads), two or four when the rows would leave threads idle.
 // Double and double-double: G lanes per row, so that a load instruction
@@ -637,12 +638,8 @@ struct tail_shape {
   static const int R = N::tr::limbs == 1 ? (N::is_complex ? 2 : 4) : (N::is_complex ? 1 : 2);
 };
 template <class N>
-__device__ void block_tail_update(int n, int degp1, int i, const double *mat, double *rhs, const double *x) {
+__device__ void block_tail_update(int n, int rows, const double *A, double *b, const double *x) {
   typedef typename N::T T;
-  const long nn = (long)n * n;
-  const int rows = (degp1 - i) * n;
-  const double *A = mat + nn * N::width;       // row r of A_1, A_2, ...
-  double *b = rhs + (long)i * n * N::width;    // its entry of b_i, b_{i+1}, ...
   if constexpr (N::tr::limbs > 2) {
     const int G = rows * 4 <= (int)blockDim.x ? 4 : (rows * 2 <= (int)blockDim.x ? 2 : 1);
     const int grp = threadIdx.x / G, part = threadIdx.x % G, ngrp = blockDim.x / G;

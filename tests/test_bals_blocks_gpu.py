@@ -5,8 +5,9 @@ test_dense_gpu.py (1e4 eps max(1, |x|) per block), at the edges: the smallest
 and largest dimension, dimensions off the tiles of 16 and 32 rows and one
 more than 32 columns, a tail one stage past a block of 4, 8, 16 and two of
 16, a skipped stage inside a block, and the rows that the digits cannot hold
-(limbs that overlap, entries near the ends of the range), which take the
-FP64 products."""
+(limbs that overlap, entries near the ends of the range) or that are too far
+above the sums they enter (unknowns in other units, sparse rows), which take
+the quad-double products."""
 import numpy as np
 import pytest
 
@@ -58,6 +59,63 @@ def test_blocked_tail_special_rows(kind):
         rhs *= 2.0 ** 310
     else:
         mat[2, 3] *= 2.0 ** -310
+    sol, fl, so, flo = solve_both(mat.reshape(-1), rhs.reshape(-1), n, degp1, szt)
+    assert np.array_equal(fl, flo)
+    assert check_bals(sol, so, 4, False, degp1, n)
+
+
+def graded(n):
+    """Powers of two 2^0, 2^60 for the unknowns, in no order."""
+    g = np.random.default_rng(n).permutation(np.arange(n) % 2 * 60)
+    return 2.0 ** g
+
+
+@pytest.mark.parametrize("n,szt,degp1", [(32, 8, 9), (40, 20, 18), (64, 16, 20)])
+def test_blocked_tail_other_units(n, szt, degp1):
+    """The unknowns in other units (columns of every A_k times 2^-g, unknowns
+    times 2^g): large entries meet small ones in every sum.  Every unknown has
+    to be as exact in its own unit as in the plain system, by the tolerance
+    above."""
+    mat, rhs = inputs(n + degp1, n, degp1)
+    mat *= 2.0 ** -np.arange(degp1)[:, None, None, None]
+    d = graded(n)
+    plain = solve_both(mat.reshape(-1), rhs.reshape(-1), n, degp1, szt)[0].reshape(degp1, n, 4)
+    sol, fl, so, flo = solve_both((mat / d[:, None]).reshape(-1), rhs.reshape(-1), n, degp1, szt)
+    assert np.array_equal(fl, flo)
+    sol, so = sol.reshape(degp1, n, 4) / d[:, None], so.reshape(degp1, n, 4) / d[:, None]
+    assert check_bals(sol.reshape(-1), so.reshape(-1), 4, False, degp1, n)
+    assert check_bals(plain.reshape(-1), so.reshape(-1), 4, False, degp1, n)
+
+
+def test_a_plain_system_takes_the_digits():
+    """Every quad-double operation of the solve commutes with a change of the
+    unknowns' units, so solutions that differ in their last bits show that the
+    plain system took the digit products, which the other cannot.  (A_0
+    dominant: the solution does not grow from stage to stage, so that what
+    the blocks subtract is not lost behind what is subtracted after them.)"""
+    n, szt, degp1 = 64, 16, 20
+    mat, rhs = inputs(1, n, degp1)
+    mat[0, range(n), range(n), 0] += 24.0
+    d = graded(n)
+    plain = solve_both(mat.reshape(-1), rhs.reshape(-1), n, degp1, szt)[0].reshape(degp1, n, 4)
+    sol, _, so, _ = solve_both((mat / d[:, None]).reshape(-1), rhs.reshape(-1), n, degp1, szt)
+    sol, so = sol.reshape(degp1, n, 4) / d[:, None], so.reshape(degp1, n, 4) / d[:, None]
+    assert check_bals(sol.reshape(-1), so.reshape(-1), 4, False, degp1, n)
+    assert check_bals(plain.reshape(-1), so.reshape(-1), 4, False, degp1, n)
+    assert np.array_equal(plain[0], sol[0]) and not np.array_equal(plain[5:], sol[5:])
+
+
+def test_blocked_tail_sparse_rows():
+    # rows of zeros, and rows of one entry (some of whose unknowns are far
+    # below the largest: a few sums of a warp by quad-double products)
+    n, szt, degp1 = 48, 16, 14
+    mat, rhs = inputs(3, n, degp1)
+    mat *= 2.0 ** -np.arange(degp1)[:, None, None, None]
+    keep = mat.copy()
+    mat[1:, ::6] = 0.0
+    mat[1:, 3::6] = 0.0
+    for k in range(1, degp1):
+        mat[k, 3::6, (5 * k) % n] = keep[k, 3::6, (5 * k) % n]
     sol, fl, so, flo = solve_both(mat.reshape(-1), rhs.reshape(-1), n, degp1, szt)
     assert np.array_equal(fl, flo)
     assert check_bals(sol, so, 4, False, degp1, n)
