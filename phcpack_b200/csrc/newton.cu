@@ -115,19 +115,29 @@ int newton_step(int prec, int cplx, int nsys, int dim, int deg, int maxdeg, int 
   double *sol = p;  p += (long)nsys * n1 * dim * W;
   double *bw = p;
   const int T = 256;
-  // at the full degree the series are contiguous already: no packing (three
-  // launches of the seven of a step on one small system)
+  // At the full degree the series are contiguous already: no packing (three
+  // launches of the seven of a step on one small system).  Constants and
+  // coefficients that do not lie on the 16 bytes that the evaluation loads at
+  // once are packed all the same (the series themselves have to lie there for
+  // the update), and so are coefficients of no monomials, which need not exist.
+  auto in_place = [&](const double *q) {
+    return deg == maxdeg && ((W & 1) || (reinterpret_cast<unsigned long long>(q) & 15) == 0);
+  };
   const double *ecst = cst, *ecff = cff, *ein = series;
   if (deg < maxdeg) {
     k_pack_series<<<grid_for((long)nsys * dim * n1 * W, T), T, 0, st>>>((long)nsys * dim, (int)W, deg, maxdeg, series, xin);
-    k_pack_series<<<grid_for((long)nsys * dim * n1 * W, T), T, 0, st>>>((long)nsys * dim, (int)W, deg, maxdeg, cst, cs);
-    if (nmon > 0)
-      k_pack_series<<<grid_for(nmon * n1 * W, T), T, 0, st>>>(nmon, (int)W, deg, maxdeg, cff, cf);
-    PHC_CHECK_LAUNCH();
-    ecst = cs;
-    ecff = cf;
     ein = xin;
   }
+  if (!in_place(cst)) {
+    k_pack_series<<<grid_for((long)nsys * dim * n1 * W, T), T, 0, st>>>((long)nsys * dim, (int)W, deg, maxdeg, cst, cs);
+    ecst = cs;
+  }
+  if (nmon == 0 || !in_place(cff)) {
+    if (nmon > 0)
+      k_pack_series<<<grid_for(nmon * n1 * W, T), T, 0, st>>>(nmon, (int)W, deg, maxdeg, cff, cf);
+    ecff = cf;
+  }
+  PHC_CHECK_LAUNCH();
   int rc = system_evaldiff(prec, cplx, nsys, dim, deg, maxvar, mon_off, nvr, idx, exps, ecst, ecff, ein, out, st);
   if (rc) return rc;
   k_linearize<<<grid_for((long)nsys * dim * (dim + 1) * n1, T), T, 0, st>>>(nsys, dim, deg, (int)W, out, jac, rhs, sol);
