@@ -37,10 +37,10 @@ int phc_abi_version(void);
  * counterpart in the reference, whose launch shapes are fixed at compile
  * time or passed per call.
  *   knob 0: polynomials (warps) per CTA of phc_system_evaldiff, 1..8
- *           (the rule: min(dim, 8), fewer when the scratch needs it; a
- *           batch of at most 1184 polynomials (296 of one-variable
- *           monomials) takes a CTA per polynomial instead, its monomials
- *           shared by the warps);
+ *           (the rule: min(dim, 8), as 8 gives; always fewer when the
+ *           scratch needs it).  A batch of at most 1184 polynomials (296 of
+ *           one-variable monomials) takes a CTA per polynomial instead, its
+ *           monomials shared by the warps, and does not depend on it;
  *   knob 1: variant of the split tracker's kernel, 1 the 64-register one
  *           (8 paths per SM), 2 the 72-register one (7 paths per SM; the
  *           128-register one when the batch or knob 2 asks for no more than

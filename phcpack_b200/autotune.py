@@ -3,7 +3,8 @@
 Three choices are swept once per shape and cached for the process:
 
 * the warps (polynomials) per CTA of ``phc_system_evaldiff`` (knob 0 of
-  ``phc_tune_set``), over 1, 2, 4 and 8;
+  ``phc_tune_set``), over 1, 2, 4 and 8, of which 8 is the built-in rule
+  (a batch of so few polynomials that each takes a CTA does not depend on it);
 * the tile size ``szt`` of the blocked QR / least squares
   (``phc_bals_solve``), over the divisors of the dimension among
   8, 16, 32 and 64 (a call argument, returned to the caller), with the
@@ -14,7 +15,8 @@ Three choices are swept once per shape and cached for the process:
   together with the paths tracked at once per SM (knob 2), 4 to 8.
 
 Every candidate is timed with CUDA events on the caller's stream after one
-untimed run; the fastest is kept (ties to the built-in rule's choice).  The
+untimed run; the fastest is kept (ties, for knob 0 all within 5 %, to the
+built-in rule's choice: the knob stays set for other shapes).  The
 knobs change launch shapes only: results are the same for every choice
 (the tests check this).
 """
@@ -57,17 +59,20 @@ def _time(torch, stream, fn, reps: int = 3) -> float:
 def tune_eval_warps(torch, stream, args, dim: int, key=None, reps: int = 3) -> dict:
     """Sweep the warps per CTA of phc_system_evaldiff; args: the argument
     tuple of the call (device pointers, the stream last).  Sets knob 0 to the
-    fastest and returns {"choice", "seconds": {warps: s}}."""
+    fastest, or to 8, the built-in rule for every dimension, unless another is
+    5 % faster, and returns {"choice", "seconds": {warps: s}}."""
     key = ("eval", key if key is not None else dim)
     if key in _cache:
         set_knob(KNOB_EVAL_WARPS, _cache[key]["choice"])
         return _cache[key]
-    cands = [w for w in (1, 2, 4, 8) if w <= max(1, dim)]
+    cands = [w for w in (1, 2, 4) if w < dim] + [8]
     secs = {}
     for w in cands:
         set_knob(KNOB_EVAL_WARPS, w)
         secs[w] = _time(torch, stream, lambda: _lib.call("phc_system_evaldiff", *args), reps)
     best = min(cands, key=lambda w: (secs[w], -w))
+    if secs[best] > 0.95 * secs[8]:
+        best = 8
     set_knob(KNOB_EVAL_WARPS, best)
     _cache[key] = {"choice": best, "seconds": secs}
     return _cache[key]

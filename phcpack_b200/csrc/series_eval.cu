@@ -149,7 +149,6 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
   const bool big = deg > 31;  // series longer than a warp
   const long series = (long)S * sizeof(double);
   const long xs = (long)((dim * S + 1) & ~1) * sizeof(double);
-  const int tuned = tune_get(kTuneEvalWarps);  // warps per CTA chosen by the autotuner
   // The squares of the variables beside the inputs, for short series, while
   // two CTAs of the built-in shape still share an SM (1024 systems n = 32
   // with exponents up to 3: one in nine products saved, 24.2 -> 22.2 ms;
@@ -160,9 +159,11 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
   // A warp per polynomial leaves most of the GPU idle on a few systems, and
   // each warp's products follow one another.  While the polynomials are
   // fewer than kSplitPolys a CTA takes one polynomial and shares its
-  // monomials among its warps, when the rows fit in shared memory.
+  // monomials among its warps, when the rows fit in shared memory.  (Whatever
+  // knob 0 says: it sizes the CTAs of the other arrangement, and what was
+  // found for a large batch must not send the small ones there.)
   const bool short_work = maxvar == 1 || (maxvar == 2 && N::tr::limbs == 1);
-  if (tuned == 0 && (long)nsys * dim <= (short_work ? kSplitPolysShort : kSplitPolys)) {
+  if ((long)nsys * dim <= (short_work ? kSplitPolysShort : kSplitPolys)) {
     const long per_warp = (warp_slots(maxvar) + maxvar + 1) * series;
     const long rows = (long)(((dim + 1) * S + 1) & ~1) * sizeof(double);
     int nw = kMaxWarpsPerBlock;
@@ -186,6 +187,7 @@ static int launch_system(int nsys, int dim, int deg, int maxvar, const int *mon_
   // shared memory when they fit beside the scratch
   const long per_warp = (warp_slots(maxvar) + (big ? 1 : 0)) * series;
   int wpb = dim < kMaxWarpsPerBlock ? dim : kMaxWarpsPerBlock;
+  const int tuned = tune_get(kTuneEvalWarps);  // warps per CTA chosen by the autotuner
   if (tuned > 0) wpb = tuned < dim ? tuned : dim;
   while (wpb > 1 && (long)wpb * per_warp > kMaxSmem) --wpb;
   const long scr = (long)wpb * per_warp;

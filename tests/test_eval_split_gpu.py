@@ -12,7 +12,7 @@ import pytest
 
 from mdcheck import abs_batch, check_scaled
 from oracle import pyoracle
-from phcpack_b200 import _lib, series
+from phcpack_b200 import _lib, autotune, series
 from phcpack_b200 import workloads as wl
 
 pytestmark = pytest.mark.gpu
@@ -20,15 +20,57 @@ ORC = pyoracle.oracle()
 RTOL = {1: 1e-14, 2: 1e-28, 4: 1e-60}
 
 
+def repeated(b):
+    """The systems of b over again, until a CTA per polynomial is too many."""
+    c = 1184 // (b.nsys * b.dim) + 1
+    nm = len(b.nvr)
+    off = np.concatenate([b.mon_off[:-1] + np.int32(i * nm) for i in range(c)] + [np.array([c * nm], np.int32)])
+    tile = lambda a: np.tile(a, (c,) + (1,) * (a.ndim - 1))
+    return c, wl.SystemBatch(c * b.nsys, b.dim, b.deg, b.maxvar, b.prec, b.cplx, off.astype(np.int32), tile(b.nvr),
+                             tile(b.idx), tile(b.exps), tile(b.cst), tile(b.cff), tile(b.input))
+
+
 def evaluate(b, knob):
+    """knob 0: a CTA per polynomial.  Otherwise that many polynomials per CTA,
+    a warp each; all copies of the systems have to agree."""
     import torch
+    copies, batch = (1, b) if knob == 0 else repeated(b)
     _lib.call("phc_tune_set", 0, knob)
     try:
-        out = series.DeviceBatch(b).evaldiff()
+        out = series.DeviceBatch(batch).evaldiff()
         torch.cuda.synchronize()
     finally:
         _lib.call("phc_tune_set", 0, 0)
-    return out.cpu().numpy()
+    out = out.cpu().numpy().reshape(copies, -1)
+    assert np.array_equal(out, np.broadcast_to(out[0], out.shape), equal_nan=True)
+    return out[0]
+
+
+@pytest.mark.parametrize("prec,cplx", [(1, True), (2, False), (4, False)])
+def test_polynomials_per_cta_agree(prec, cplx):
+    # bit for bit: the same products, summed in the same order
+    b = wl.eval_batch(29, 3, 11, 14, 10, 4, prec, cplx, expmax=3)
+    out = [evaluate(b, knob) for knob in (1, 2, 4, 8)]
+    for o in out[1:]:
+        assert np.array_equal(o, out[0])
+
+
+def test_few_polynomials_do_not_depend_on_the_knob():
+    """The warps per CTA that the autotuner found for a large batch do not
+    take the arrangement for few polynomials away from a small one: 8
+    polynomials of 12 monomials take at most half as long again as by the
+    built-in rule (a warp per polynomial: five times as long)."""
+    import torch
+    db = series.DeviceBatch(wl.eval_batch(5, 1, 8, 15, 12, 4, 2, True, expmax=2))
+    stream = torch.cuda.current_stream()
+    secs = {}
+    try:
+        for knob in (0, 2, 8):
+            _lib.call("phc_tune_set", 0, knob)
+            secs[knob] = min(autotune._time(torch, stream, db.evaldiff, reps=9) for _ in range(3))
+    finally:
+        _lib.call("phc_tune_set", 0, 0)
+    assert max(secs.values()) <= 1.5 * secs[0], secs
 
 
 @pytest.mark.parametrize("prec,cplx,nsys,dim,deg,nmon,maxvar", [
