@@ -49,27 +49,28 @@ __device__ __forceinline__ void stage_inputs(const double *__restrict__ xin, dou
 // The squares of the variables that have an exponent above 2 in the monomials
 // m0..m1-1, into sq (dim series): a product each, one less wherever they
 // occur.  X in shared memory.  Called by the whole CTA; the caller
-// synchronises before they are read.
+// synchronises before they are read.  (Which variables those are is marked in
+// the squares' own places: static shared memory would count against the
+// launches without squares too, whose scratch may take all there is.)
 template <class N, bool BIG>
 __device__ const double *needed_squares(int dim, int deg, int maxvar, int m0, int m1, const int *__restrict__ nvr,
                                         const int *__restrict__ idx, const int *__restrict__ exps, const double *X,
                                         double *sq) {
-  __shared__ unsigned need[kSquareDims / 32];
-  if (threadIdx.x < kSquareDims / 32) need[threadIdx.x] = 0u;
+  const int S = (deg + 1) * N::width;
+  for (int i = threadIdx.x; i < dim; i += blockDim.x) sq[i * S] = 0.0;
   __syncthreads();
   for (int m = m0 + threadIdx.x; m < m1; m += blockDim.x) {
     const int k = nvr[m];
     if (k < 1 || k > maxvar) continue;
     for (int v = 0; v < k; ++v) {
       const int i = idx[(long)m * maxvar + v];
-      if (i >= 0 && i < dim && exps[(long)m * maxvar + v] > 2) atomicOr(&need[i >> 5], 1u << (i & 31));
+      if (i >= 0 && i < dim && exps[(long)m * maxvar + v] > 2) sq[i * S] = 1.0;
     }
   }
   __syncthreads();
-  const int S = (deg + 1) * N::width;
   const typename wser<N, BIG>::map map(deg, threadIdx.x & 31, 0);
   for (int i = threadIdx.x >> 5; i < dim; i += blockDim.x >> 5) {
-    if (!((need[i >> 5] >> (i & 31)) & 1u)) continue;
+    if (sq[i * S] == 0.0) continue;
     const typename N::T z = wser<N, BIG>::conv(X + i * S, X + i * S, map);
     if (map.valid) md::stn(sq + i * S + map.kout() * N::width, z);
   }

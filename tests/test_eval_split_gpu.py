@@ -96,3 +96,12 @@ def test_squares_match_oracle(prec, cplx, dim, deg, expmax):
     scale = ORC.system_evaldiff(abs_batch(b))
     for knob in (2, 8):
         assert check_scaled(evaluate(b, knob), ref, scale, prec, cplx, RTOL[prec]) <= 1.0
+
+
+def test_scratch_that_takes_all_shared_memory():
+    # degree 148, 20 variables, double: five warps' scratch is 8 bytes short
+    # of the 227 KB a CTA can have
+    b = wl.eval_batch(21, 60, 20, 148, 2, 20, 1, False, minvar=18)
+    out = series.DeviceBatch(b).evaldiff().cpu().numpy()
+    scale = ORC.system_evaldiff(abs_batch(b))
+    assert check_scaled(out, ORC.system_evaldiff(b), scale, 1, False, RTOL[1]) <= 1.0
