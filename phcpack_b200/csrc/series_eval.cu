@@ -48,7 +48,10 @@ __device__ __forceinline__ void stage_inputs(const double *__restrict__ xin, dou
 
 // The squares of the variables that have an exponent above 2 in the monomials
 // m0..m1-1, into sq (dim series): a product each, one less wherever they
-// occur.  X in shared memory.  Called by the whole CTA; the caller
+// occur.  Null when a coefficient of X (all variables, so that it does not
+// depend on the polynomials of the CTA) is below 2^-400 or above 2^500: a
+// square could leave the range, or lose lower limbs at its end, where c x x
+// does not.  X in shared memory.  Called by the whole CTA; the caller
 // synchronises before they are read.  (Which variables those are is marked in
 // the squares' own places: static shared memory would count against the
 // launches without squares too, whose scratch may take all there is.)
@@ -58,7 +61,13 @@ __device__ const double *needed_squares(int dim, int deg, int maxvar, int m0, in
                                         double *sq) {
   const int S = (deg + 1) * N::width;
   for (int i = threadIdx.x; i < dim; i += blockDim.x) sq[i * S] = 0.0;
-  __syncthreads();
+  __syncthreads();  // and X is in place
+  bool outside = false;
+  for (int i = threadIdx.x; i < dim * (deg + 1) * (N::width / N::tr::limbs); i += blockDim.x) {
+    const double a = fabs(X[i * N::tr::limbs]);
+    outside = outside || !(a == 0.0 || (a >= 0x1p-400 && a <= 0x1p500));
+  }
+  if (__syncthreads_or(outside)) return nullptr;
   for (int m = m0 + threadIdx.x; m < m1; m += blockDim.x) {
     const int k = nvr[m];
     if (k < 1 || k > maxvar) continue;

@@ -105,3 +105,22 @@ def test_scratch_that_takes_all_shared_memory():
     out = series.DeviceBatch(b).evaldiff().cpu().numpy()
     scale = ORC.system_evaldiff(abs_batch(b))
     assert check_scaled(out, ORC.system_evaldiff(b), scale, 1, False, RTOL[1]) <= 1.0
+
+
+@pytest.mark.parametrize("shift", [520, -560])
+@pytest.mark.parametrize("prec,cplx", [(1, False), (2, True), (4, False)])
+def test_squares_out_of_range(prec, cplx, shift):
+    """x_0 so large or small that its square leaves the range, with
+    coefficients that bring its powers back: c x x x is a number."""
+    b = wl.eval_batch(77, 2, 5, 9, 6, 3, prec, cplx, expmax=4)
+    b.input.reshape(2, 5, -1)[:, 0] *= 2.0 ** shift
+    e = ((b.idx == 0) & (np.arange(3) < b.nvr[:, None])) * b.exps
+    assert e.max() >= 3
+    b.exps[e == 4] = 3
+    e = np.minimum(e, 3).max(axis=1)
+    b.cff.reshape(len(e), -1)[:] *= np.where(e > 0, 2.0 ** (-np.sign(shift) * 510.0 * np.maximum(e - 1, 0)), 1.0)[:, None]
+    ref = ORC.system_evaldiff(b)
+    assert np.isfinite(ref).all()
+    scale = ORC.system_evaldiff(abs_batch(b))
+    for knob in (0, 4):
+        assert check_scaled(evaluate(b, knob), ref, scale, prec, cplx, RTOL[prec]) <= 1.0
