@@ -68,6 +68,14 @@ __global__ void __launch_bounds__(kDenseThreads, dense_many<N>::value)
   }
 }
 
+// Shared memory (doubles) of k_bals_solve behind dense_smem for what is not
+// needed at one time: the WY panels of the QR (staged), then the digits of the
+// blocked tail.
+__host__ __device__ inline long bals_scratch(int n, int szt, int W, bool stage, bool blocked) {
+  const long wy = stage ? 4L * n * szt * W : 0, digits = blocked ? kI8Smem / (long)sizeof(double) : 0;
+  return wy > digits ? wy : digits;
+}
+
 // Block lower-triangular Toeplitz least squares, one instance per CTA:
 // Newton/dbl2_bals_kernels.cu:554 (GPU_dbl2_bals_solve) with the head at
 // :108 and the tail at dbl2_tail_kernels.cu:154; skip rules of
@@ -95,9 +103,10 @@ __global__ void __launch_bounds__(kDenseThreads, PER_SM)
   int *fl = flags + inst * 5;
   double *wk = work + inst * dense_stride(n, szt, W, OZ);
   // staged: the WY panels, the column panel of R and then the inverted
-  // diagonal tiles of R in shared memory
+  // diagonal tiles of R in shared memory; the digits of the blocked tail take
+  // the place of the WY panels
   double *ywpt = stage ? sm + dense_smem_doubles(n, szt, W) : wk;
-  double *panel = stage ? ywpt + 4L * n * szt * W : nullptr;
+  double *panel = stage ? ywpt + bals_scratch(n, szt, W, true, blocked) : nullptr;
   double *tinv = stage ? panel : wk + 4L * n * szt * W;
   int zeroQ = fl[0], noqr = fl[1];
   const int tail0 = max(1, tailidx >= 0 ? tailidx : fl[4]);
@@ -339,13 +348,13 @@ template <class N>
 static int bals_launch(int ninst, int n, int degp1, int szt, int tailidx, const double *mat, double *rhs, double *sol,
                        double *Q, double *R, int *flags, double *work, cudaStream_t st, bool oz) {
   const int stage = dense_stage(n, szt, N::width) ? 1 : 0;
-  long smem = (stage ? dense_smem_doubles_staged(n, szt, N::width) : dense_smem_doubles(n, szt, N::width)) *
-              (long)sizeof(double);
   // real quad-double of dimension 32..64 with a tail longer than one block of
   // four: the digit products of tail_i8.cuh (their shared memory still lets
-  // two CTAs share an SM; the staged kernel has no room for it)
-  const int blocked = (N::tr::limbs == 4 && !N::is_complex && !stage && n >= kI8MinN && n <= kI8MaxN && degp1 > 5) ? 1 : 0;
-  if (blocked) smem += kI8Smem;
+  // two unstaged CTAs share an SM)
+  const int blocked = (N::tr::limbs == 4 && !N::is_complex && n >= kI8MinN && n <= kI8MaxN && degp1 > 5) ? 1 : 0;
+  // (staged: at most the 227 KB of dense_stage, or 90 KB of digits beside panels smaller than those)
+  const long smem = (dense_smem_doubles(n, szt, N::width) + bals_scratch(n, szt, N::width, stage, blocked) +
+                     (stage ? (long)n * szt * N::width : 0)) * (long)sizeof(double);
   bool many = false;
   const int rc = dense_wants_many(ninst, &many);
   if (rc) return rc;

@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 from oracle import pyoracle
-from phcpack_b200 import dense
+from phcpack_b200 import _lib, dense
 from phcpack_b200 import workloads as wl
 from test_dense_gpu import check_bals
 
@@ -119,3 +119,20 @@ def test_blocked_tail_sparse_rows():
     sol, fl, so, flo = solve_both(mat.reshape(-1), rhs.reshape(-1), n, degp1, szt)
     assert np.array_equal(fl, flo)
     assert check_bals(sol, so, 4, False, degp1, n)
+
+
+@pytest.mark.parametrize("n,szt,degp1", [(36, 4, 10), (64, 8, 19), (64, 16, 9)])
+def test_staged_panels_do_not_change_the_tail(n, szt, degp1):
+    # knob 3 moves panels between global and shared memory, whether the digits
+    # fit in the place of the WY panels (tile 16) or not: bit for bit the same
+    mat, rhs = inputs(n, n, degp1)
+    mat *= 2.0 ** -np.arange(degp1)[:, None, None, None]
+    out = []
+    try:
+        for stage in (1, 2):
+            _lib.call("phc_tune_set", 3, stage)
+            out.append(dense.bals_solve_host(4, False, mat.reshape(-1), rhs.reshape(-1), 1, n, degp1, szt))
+    finally:
+        _lib.call("phc_tune_set", 3, 0)
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
