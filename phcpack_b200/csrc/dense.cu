@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(kDenseThreads, PER_SM)
       }
     }
   }
+  __syncthreads();  // every thread has read the flags (a call of one stage may get here without a barrier)
   if (threadIdx.x == 0) {
     fl[0] = zeroQ;
     fl[1] = noqr;

@@ -160,3 +160,19 @@ def test_linear_residue_vs_reference(prec, cplx, tailidx):
         rows = res[q].reshape(degp1, n * W)
         assert np.array_equal(rows[:tailidx], np.asarray(prev[q]).reshape(degp1, n * W)[:tailidx])
         assert abs(mx[q, 0] - mx_ref[0]) <= 1e-12 * mx_ref[0]
+
+
+@pytest.mark.parametrize("prec,cplx", [(1, False), (2, True), (4, False)])
+def test_bals_one_stage_with_a_zero_right_hand_side(prec, cplx):
+    """degp1 = 1, zeroQ = 0 and right hand sides below the skip threshold:
+    every entry of the solutions (more of them than a warp's lanes, stale on
+    entry) is set to zero and noqr to 1, in every instance."""
+    n, ninst = 70, 64
+    W = dense.width(prec, cplx)
+    rng = np.random.default_rng(1)
+    mat = batch_of([wl.random_numbers(rng, (1, n, n), prec, cplx, "normal") for _ in range(ninst)])
+    rhs = np.full(ninst * n * W, 1e-80 if prec > 1 else 1e-18)
+    sol, _, _, _, fl = dense.bals_solve_host(prec, cplx, mat, rhs, ninst, n, 1, 35, sol=np.ones(ninst * n * W),
+                                             flags=np.tile(np.array([0, 0, 0, 0, 1], np.int32), ninst))
+    assert np.array_equal(fl.reshape(ninst, 5)[:, :2], np.tile([0, 1], (ninst, 1)))
+    assert not sol.any()
