@@ -49,8 +49,8 @@ __global__ void __launch_bounds__(kDenseThreads, PER_SM)
 // Like Matrices/dbl2_tabs_kernels.cu:952 (GPU_dbl2_upper_tiled_solver): b is
 // overwritten by the updated right hand sides and the diagonal tiles of U by
 // their inverses.
-template <class N>
-__global__ void __launch_bounds__(kDenseThreads, dense_many<N>::value)
+template <class N, int PER_SM>
+__global__ void __launch_bounds__(kDenseThreads, PER_SM)
     k_upper_tiled_solver(int dim, int szt, double *__restrict__ U, double *__restrict__ b, double *__restrict__ x,
                          double *__restrict__ work) {
   const int W = N::width;
@@ -340,7 +340,13 @@ static int residue_launch(int ninst, int n, int degp1, int tailidx, const double
 
 template <class N>
 static int tabs_launch(int ninst, int dim, int szt, double *U, double *b, double *x, double *work, cudaStream_t st) {
-  k_upper_tiled_solver<N><<<ninst, kDenseThreads, 0, st>>>(dim, szt, U, b, x, work);
+  bool many = false;
+  const int rc = dense_wants_many(ninst, &many);
+  if (rc) return rc;
+  // (1000 systems of dimension 60, double-double: 57 us at four per SM, 81 at
+  // two; 50 of dimension 40, complex double-double: 23 at three, 21 at two)
+  auto kern = many ? k_upper_tiled_solver<N, dense_many<N>::value> : k_upper_tiled_solver<N, kDenseFew>;
+  kern<<<ninst, kDenseThreads, 0, st>>>(dim, szt, U, b, x, work);
   PHC_CHECK_LAUNCH();
   return PHC_OK;
 }
