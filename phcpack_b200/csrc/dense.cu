@@ -240,8 +240,10 @@ static int qr_launch(int ninst, int n, int ncols, int szt, const double *A, doub
   bool many = false;
   const int rc = dense_wants_many(ninst, &many);
   if (rc) return rc;
-  const int kMany = dense_many<N>::value;
-  auto kern = oz ? (many ? k_blocked_houseqr<N, true, kMany> : k_blocked_houseqr<N, true, kDenseFew>)
+  // (with the tensor-core products double-double spills at four per SM: 600
+  // instances of dimension 64 3.20 ms, 3.10 at two; double 1.17 and 1.23)
+  const int kMany = dense_many<N>::value, kManyOz = N::tr::limbs == 1 ? kMany : kDenseFew;
+  auto kern = oz ? (many ? k_blocked_houseqr<N, true, kManyOz> : k_blocked_houseqr<N, true, kDenseFew>)
                  : (many ? k_blocked_houseqr<N, false, kMany> : k_blocked_houseqr<N, false, kDenseFew>);
   PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<ninst, kDenseThreads, smem, st>>>(n, ncols, szt, A, Q, R, work, stage);
