@@ -197,12 +197,14 @@ __device__ __forceinline__ void dot_acc(md::msum<N> &sum, const double *a, long 
 // norm's reduction, and the warps 0 and 1 form beta and 1/v0 side by side.
 // Four barriers per column.
 //
-// Everything is formed with the column scaled by 2^-E, the power of two above
-// the largest x_i below the diagonal (exact, no other bits away from the ends
-// of the range): unscaled, sigma and the D_j lose their lower limbs, and 1/v0
-// overflows, where small x_i stand below an x0 of order one.  A column is
-// left alone (beta = 0) where the reference's beta is zero: when the squares
-// of all x_i underflow, or the square of v0 does.
+// Where sigma or x0 is near an end of the range the first sweep is done again
+// with the column scaled by 2^-E, the power of two above the largest x_i below
+// the diagonal (exact): unscaled, sigma and the D_j lose their lower limbs,
+// and 1/v0 overflows, where small x_i stand below an x0 of order one.  (All
+// columns scaled gives the same bits, at 5 to 10 % of a double or
+// double-double QR.)  A column is left alone (beta = 0) where the reference's
+// beta is zero: when the squares of all x_i underflow, or the square of v0
+// does.
 //
 // Entry (i, j) of R sits at Rm[(i - r0) * ld + (j - c0)]: the whole matrix
 // (r0 = c0 = 0, ld = ncols) or a panel of it staged in shared memory.  Leaves
@@ -243,6 +245,32 @@ __device__ __forceinline__ md::cx<R> mul_pow2(const md::cx<R> &a, double s) {
   return r;
 }
 
+// D_j for the nc columns from col's on, rows 1..m-1 of col, into w (D_0 =
+// sigma); SCALED: with x 2^-E for x, down = 2^-E.  4 lanes per column, 8 when
+// the columns are few and long.
+template <class N, bool SCALED>
+__device__ __forceinline__ void reflect_sums(int m, int nc, long ld, const double *col, double *w, double down) {
+  typedef typename N::T T;
+  const int G = (nc * 8 <= (int)blockDim.x && m > 16) ? 8 : 4;
+  const int grp = threadIdx.x / G, part = threadIdx.x % G, ngrp = blockDim.x / G;
+  for (int base = 0; base < nc; base += ngrp) {
+    const int j = base + grp;
+    md::msum<N> sum;
+    sum.zero();
+    if (j < nc)
+      for (int i = 1 + part; i < m; i += G) {
+        T x = ldn_at<N>(col, (long)i * ld), r = ldn_at<N>(col, (long)i * ld + j);
+        if (SCALED) {
+          x = mul_pow2(x, down);
+          if (j == 0) r = x;
+        }
+        sum.cfma(r, x);
+      }
+    const T d = group_sum<N>(sum.value(), G);
+    if (j < nc && part == 0) stn_at<N>(w, j, d);
+  }
+}
+
 template <class N>
 __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_smem &S, int r0, int c0) {
   typedef typename N::T T;
@@ -250,30 +278,19 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
   typedef md::num<R, false> RN;
   const int m = n - c, nc = e - c;
   double *col = Rm + ((long)(c - r0) * ld + (c - c0)) * N::width;  // entry (c, c)
-  // the scale, by every warp for itself
-  unsigned mx = 0u;
-  for (int i = 1 + (threadIdx.x & 31); i < m; i += 32) mx = max(mx, lead_word<N>(col, (long)i * ld));
-  const int E = reflect_exponent(__reduce_max_sync(0xffffffffu, mx), lead_word<N>(col, 0));
-  const double down = pow2(-E);
-  {
-    // D_j for the panel's columns, 4 lanes per column (8 when the columns
-    // are few and long)
-    const int G = (nc * 8 <= (int)blockDim.x && m > 16) ? 8 : 4;
-    const int grp = threadIdx.x / G, part = threadIdx.x % G, ngrp = blockDim.x / G;
-    for (int base = 0; base < nc; base += ngrp) {
-      const int j = base + grp;
-      md::msum<N> sum;
-      sum.zero();
-      if (j < nc)
-        for (int i = 1 + part; i < m; i += G) {
-          const T x = mul_pow2(ldn_at<N>(col, (long)i * ld), down);
-          sum.cfma(j == 0 ? x : ldn_at<N>(col, (long)i * ld + j), x);
-        }
-      const T d = group_sum<N>(sum.value(), G);
-      if (j < nc && part == 0) stn_at<N>(S.w, j, d);
-    }
-  }
+  reflect_sums<N, false>(m, nc, ld, col, S.w, 1.0);
   __syncthreads();
+  int E = 0;
+  const double sig = N::re_lead(ldn_at<N>(S.w, 0));
+  if (m > 1 && !(sig >= 0x1p-120 && sig <= 0x1p600 && N::lead(ldn_at<N>(col, 0)) <= 0x1p400)) {
+    unsigned mx = 0u;  // the scale, by every warp for itself
+    for (int i = 1 + (threadIdx.x & 31); i < m; i += 32) mx = max(mx, lead_word<N>(col, (long)i * ld));
+    E = reflect_exponent(__reduce_max_sync(0xffffffffu, mx), lead_word<N>(col, 0));
+    __syncthreads();  // every thread has read S.w
+    if (E != 0) reflect_sums<N, true>(m, nc, ld, col, S.w, pow2(-E));
+    __syncthreads();
+  }
+  const double down = pow2(-E);
   const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   if (warp < 2) {
     const T x0 = mul_pow2(ldn_at<N>(col, 0), down);
@@ -331,13 +348,13 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
         T v = N::one();
         if (t > 0) {
           v = ldn_at<N>(col, (long)t * ld);
-          if (!trivial) v = N::mul(mul_pow2(v, down), inv);
+          if (!trivial) v = N::mul(E != 0 ? mul_pow2(v, down) : v, inv);
         }
         stn_at<N>(S.v, t, v);
       } else if (!trivial) {
         const int j = t - m;
         const T dj = ldn_at<N>(S.w, j);  // D_j 2^-E, at j = 0 sigma 4^-E
-        const T d = md::mul_add<N>(N::conj(ldn_at<N>(col, j)), inv, j == 0 ? mul_pow2(dj, pow2(E)) : dj);
+        const T d = md::mul_add<N>(N::conj(ldn_at<N>(col, j)), inv, j == 0 && E != 0 ? mul_pow2(dj, pow2(E)) : dj);
         stn_at<N>(S.w, j, N::scale(d, beta));
       }
     }
