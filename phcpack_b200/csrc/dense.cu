@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(kDenseThreads, PER_SM)
 // Stage the WY panels and the column panel of R in shared memory?  Only on
 // request (knob 3 of phc_tune_set = 2) and when they fit: the staged kernel
 // runs one CTA per SM where the unstaged one runs two, and on the
-// quad-double least squares of dimension 64 it measured twice as slow at
-// tile 16 (53.6 against 26.0 ms for 512 instances) and no faster at others;
+// quad-double least squares of dimension 64 it measured half as slow again at
+// tile 16 (40.0 against 27.4 ms for 512 instances) and no faster at others;
 // the autotuner times both.
 static bool dense_stage(int n, int szt, int W) {
   const long staged = dense_smem_doubles_staged(n, szt, W) * (long)sizeof(double);

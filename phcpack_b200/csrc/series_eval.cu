@@ -14,8 +14,8 @@
 // (n = 32, 32 monomials, degree 31, complex double-double): 37.4 ms with the
 // multiple-double operators, 29.9 with open accumulators (md::macc), 28.5
 // with two-variable monomials in three products instead of four, 24.2 with
-// one inlined product per kernel in chunks of three terms: 70 % of the FP64
-// pipe's rate.  At 16 warps per SM; 24 (80 registers) measured 4 % slower, 8
+// one inlined product per kernel in chunks of three terms, 22.0 with the
+// squares of the variables at hand: 77 % of the FP64 pipe's rate.  At 16 warps per SM; 24 (80 registers) measured 4 % slower, 8
 // with 153 registers 25 %.
 #include "common.cuh"
 #include "series_eval.cuh"

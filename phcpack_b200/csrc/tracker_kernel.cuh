@@ -572,9 +572,10 @@ static int track_launch(const TrackDev &S, const TrackParDev &P, int nmono_max, 
   if constexpr (track_min_blocks<PN, RN, kTrackWide>::split) {
     // one wave at a lower occupancy: take the variant with more registers
     // (the autotuner's choice when it made one: 1 narrow, 2 wide).  On the
-    // dense quadratic n = 10 homotopy: 1024 paths 10.3 ms at 7 per SM against
-    // 12 ms at 4 (two waves); 500 paths 6.1 ms at 4 against 7.0 at 7; one
-    // path 3.5 against 4.1.
+    // dense quadratic n = 10 homotopy, plain step: 1024 paths 13.0 ms at 7 per
+    // SM against 14.7 at 4 (two waves) and 15.5 with 64 registers; 500 paths
+    // 8.6 ms with 128 registers against 11.8 with 64; one path 4.1 against
+    // 5.6.
     auto wide = k_track<PN, CN, RN, kTrackWide>;
     auto few = k_track<PN, CN, RN, kTrackFew>;
     PHC_CUDA(cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
