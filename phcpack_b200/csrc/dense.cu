@@ -222,12 +222,12 @@ static bool dense_stage(int n, int szt, int W) {
   return tune_get(kTuneDenseStage) == 2 && staged <= 227L * 1024 - 1024;
 }
 
-// More than two instances per SM of the current device?
-static int dense_wants_many(int ninst, bool *many) {
+// More than per_sm instances per SM of the current device?
+static int dense_wants_many(int ninst, bool *many, int per_sm = kDenseFew) {
   int dev = 0, nsm = 148;
   PHC_CUDA(cudaGetDevice(&dev));
   PHC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  *many = (long)ninst > (long)kDenseFew * nsm;
+  *many = (long)ninst > (long)per_sm * nsm;
   return PHC_OK;
 }
 
@@ -240,10 +240,16 @@ static int qr_launch(int ninst, int n, int ncols, int szt, const double *A, doub
   bool many = false;
   const int rc = dense_wants_many(ninst, &many);
   if (rc) return rc;
-  // (with the tensor-core products double-double spills at four per SM: 600
-  // instances of dimension 64 3.20 ms, 3.10 at two; double 1.17 and 1.23)
-  const int kMany = dense_many<N>::value, kManyOz = N::tr::limbs == 1 ? kMany : kDenseFew;
-  auto kern = oz ? (many ? k_blocked_houseqr<N, true, kManyOz> : k_blocked_houseqr<N, true, kDenseFew>)
+  // With the tensor-core products three per SM: 600 instances of dimension 64
+  // in double-double 2.77 ms, 3.02 at two, 3.12 at four, which spills; 300 in
+  // double 0.59 ms, 0.78 and 0.63, but 1000, in a third wave, 1.49 against
+  // 1.36 at four.
+  const int kMany = dense_many<N>::value, kOz = N::tr::limbs == 4 ? 2 : 3, kOzWaves = N::tr::limbs == 1 ? 4 : kOz;
+  bool waves = false;
+  if (oz && dense_wants_many(ninst, &waves, 2 * kOz)) return PHC_ERR_CUDA;
+  auto kern = oz ? (waves  ? k_blocked_houseqr<N, true, kOzWaves>
+                    : many ? k_blocked_houseqr<N, true, kOz>
+                           : k_blocked_houseqr<N, true, kDenseFew>)
                  : (many ? k_blocked_houseqr<N, false, kMany> : k_blocked_houseqr<N, false, kDenseFew>);
   PHC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<ninst, kDenseThreads, smem, st>>>(n, ncols, szt, A, Q, R, work, stage);
