@@ -515,9 +515,8 @@ template <class R> struct num<R, true> {
 // Errors: dd (u = 2^-53; root mean square over random dot products of 1..192
 // terms, equal and graded magnitudes) 0.20-0.69 u^2 sum |ab| against
 // 0.33-1.16 for rounding after every operation, equal (0.47) for one or two
-// terms; qd (largest over 4000 sums each) 0.12 2^-212 sum |ab| against 0.12
-// for random products, 0.12 against 0.24 and 0.03 against 0.14 for sums whose
-// terms cancel at one or several limbs.
+// terms; qd (largest over 330,000 sums whose terms cancel at one or several
+// limbs) 0.12 2^-212 sum |ab| against 0.24, equal (0.12) for random products.
 template <class R> struct macc;
 template <> struct macc<double> {
   double s;
@@ -604,13 +603,14 @@ template <> struct macc<qd> {
     // behind them, and renorm5 takes the larger of two numbers first.  One
     // pass of error-free sums brings the sum's leading part to the front but
     // leaves its errors in no order (1 % of the sums with a term that cancels
-    // down to its second limb lost half their digits), a second one orders
-    // them.
+    // down to its second limb lost half their digits); the middle three are
+    // ordered once more.  (The last one is below the precision, the first
+    // above all.)
     double e[5] = {f0, f1, f2, f3, f4};
 #pragma unroll
-    for (int pass = 0; pass < 2; ++pass)
+    for (int i = 3; i >= 0; --i) e[i] = two_sum(e[i], e[i + 1], e[i + 1]);
 #pragma unroll
-      for (int i = 3; i >= 0; --i) e[i] = two_sum(e[i], e[i + 1], e[i + 1]);
+    for (int i = 2; i >= 1; --i) e[i] = two_sum(e[i], e[i + 1], e[i + 1]);
     return renorm5(e[0], e[1], e[2], e[3], e[4]);
   }
 };
