@@ -271,6 +271,82 @@ __device__ __forceinline__ void reflect_sums(int m, int nc, long ld, const doubl
   }
 }
 
+// beta (into misc[0]) and 1/v0 (into misc[2]) from sigma (w[0]) and x0 by the
+// warps 0 and 1 side by side; SCALED: of the column times 2^-E.  Unscaled,
+// misc[4] says whether sigma or x0 is near an end of the range.
+template <class N, bool SCALED>
+__device__ __forceinline__ void reflect_scalars(int m, const double *col, const double *w, double *misc, int E) {
+  typedef typename N::T T;
+  typedef typename N::real R;
+  typedef md::num<R, false> RN;
+  const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  if (warp >= 2) return;
+  T x0 = ldn_at<N>(col, 0);
+  if (SCALED) x0 = mul_pow2(x0, pow2(-E));
+  R sigma;
+  {
+    const T d0 = ldn_at<N>(w, 0);
+    if constexpr (N::is_complex)
+      sigma = d0.re;
+    else
+      sigma = d0;
+  }
+  const bool do_beta = warp == 0, do_inv = warp == 1 || nwarp == 1;
+  if (!SCALED && do_beta && (threadIdx.x & 31) == 0) {
+    const double sig = md::lead(sigma);
+    misc[4 * N::width] = (m == 1 || (sig >= 0x1p-120 && sig <= 0x1p600 && N::lead(x0) <= 0x1p400)) ? 0.0 : 1.0;
+  }
+  R beta = RN::zero();
+  T inv = N::one();
+  if (!md::is_zero(sigma) && !(SCALED && md::lead(sigma) < pow2(2 * (kReflectUnder - E)))) {
+    T v0 = N::zero();
+    if constexpr (N::is_complex) {
+      const R sq0 = N::norm2(x0);
+      const R rad0 = RN::tr::sqrt(sq0);
+      R mu = RN::tr::sqrt(RN::add(sq0, sigma));
+      if (md::is_zero(rad0)) {
+        v0 = N::mkc(RN::neg(mu), RN::zero());
+      } else {
+        mu = RN::tr::div(mu, rad0);
+        v0 = N::mkc(RN::sub(x0.re, RN::mul(mu, x0.re)), RN::sub(x0.im, RN::mul(mu, x0.im)));
+      }
+      const R v0sq = N::norm2(v0);
+      const bool under = SCALED && md::lead(v0sq) < pow2(2 * (kReflectUnder - E));
+      if (do_beta && !under) beta = md::mul_d(RN::tr::div(v0sq, RN::add(sigma, v0sq)), 2.0);
+      if (do_inv) inv = N::mkc(RN::tr::div(v0.re, v0sq), RN::neg(RN::tr::div(v0.im, v0sq)));
+    } else {
+      const R mu = RN::tr::sqrt(RN::add(RN::mul(x0, x0), sigma));
+      const bool cancel = !(md::lead(x0) <= 0.0);  // x0 - mu would cancel
+      const R a = cancel ? RN::add(x0, mu) : RN::sub(x0, mu);
+      const bool under = SCALED && cancel && md::lead(sigma) < __dmul_rn(md::lead(a), pow2(kReflectUnder - E));
+      // sigma + v0^2 = -2 mu v0, so that beta = -v0 / mu: one division
+      // beside the other warp's, none of them waiting for another
+      if (do_inv) inv = cancel ? RN::neg(RN::tr::div(a, sigma)) : RN::tr::div(RN::one(), a);
+      if (do_beta && !under) beta = cancel ? RN::tr::div(sigma, RN::mul(a, mu)) : RN::neg(RN::tr::div(a, mu));
+    }
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (do_beta) stn_at<RN>(misc, 0, beta);
+    if (do_inv) stn_at<N>(misc + 2 * N::width, 0, inv);
+  }
+}
+
+// The sums and scalars again with the column's scale; returns E (0 for a
+// column of zeros below the diagonal: they stand).  Out of line: columns that
+// need it are rare, and its code would take the others' instruction cache.
+template <class N>
+__device__ __noinline__ int reflect_rescaled(int m, int nc, long ld, const double *col, double *w, double *misc) {
+  unsigned mx = 0u;  // the scale, by every warp for itself
+  for (int i = 1 + (threadIdx.x & 31); i < m; i += 32) mx = max(mx, lead_word<N>(col, (long)i * ld));
+  const int E = reflect_exponent(__reduce_max_sync(0xffffffffu, mx), lead_word<N>(col, 0));
+  if (E == 0) return 0;
+  reflect_sums<N, true>(m, nc, ld, col, w, pow2(-E));
+  __syncthreads();
+  reflect_scalars<N, true>(m, col, w, misc, E);
+  __syncthreads();
+  return E;
+}
+
 template <class N>
 __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_smem &S, int r0, int c0) {
   typedef typename N::T T;
@@ -280,64 +356,10 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
   double *col = Rm + ((long)(c - r0) * ld + (c - c0)) * N::width;  // entry (c, c)
   reflect_sums<N, false>(m, nc, ld, col, S.w, 1.0);
   __syncthreads();
-  int E = 0;
-  const double sig = N::re_lead(ldn_at<N>(S.w, 0));
-  if (m > 1 && !(sig >= 0x1p-120 && sig <= 0x1p600 && N::lead(ldn_at<N>(col, 0)) <= 0x1p400)) {
-    unsigned mx = 0u;  // the scale, by every warp for itself
-    for (int i = 1 + (threadIdx.x & 31); i < m; i += 32) mx = max(mx, lead_word<N>(col, (long)i * ld));
-    E = reflect_exponent(__reduce_max_sync(0xffffffffu, mx), lead_word<N>(col, 0));
-    __syncthreads();  // every thread has read S.w
-    if (E != 0) reflect_sums<N, true>(m, nc, ld, col, S.w, pow2(-E));
-    __syncthreads();
-  }
-  const double down = pow2(-E);
-  const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  if (warp < 2) {
-    const T x0 = mul_pow2(ldn_at<N>(col, 0), down);
-    R sigma;
-    {
-      const T d0 = ldn_at<N>(S.w, 0);
-      if constexpr (N::is_complex)
-        sigma = d0.re;
-      else
-        sigma = d0;
-    }
-    const bool do_beta = warp == 0, do_inv = warp == 1 || nwarp == 1;
-    R beta = RN::zero();
-    T inv = N::one();
-    if (!md::is_zero(sigma) && !(md::lead(sigma) < pow2(2 * (kReflectUnder - E)))) {
-      T v0 = N::zero();
-      if constexpr (N::is_complex) {
-        const R sq0 = N::norm2(x0);
-        const R rad0 = RN::tr::sqrt(sq0);
-        R mu = RN::tr::sqrt(RN::add(sq0, sigma));
-        if (md::is_zero(rad0)) {
-          v0 = N::mkc(RN::neg(mu), RN::zero());
-        } else {
-          mu = RN::tr::div(mu, rad0);
-          v0 = N::mkc(RN::sub(x0.re, RN::mul(mu, x0.re)), RN::sub(x0.im, RN::mul(mu, x0.im)));
-        }
-        const R v0sq = N::norm2(v0);
-        const bool under = md::lead(v0sq) < pow2(2 * (kReflectUnder - E));
-        if (do_beta && !under) beta = md::mul_d(RN::tr::div(v0sq, RN::add(sigma, v0sq)), 2.0);
-        if (do_inv) inv = N::mkc(RN::tr::div(v0.re, v0sq), RN::neg(RN::tr::div(v0.im, v0sq)));
-      } else {
-        const R mu = RN::tr::sqrt(RN::add(RN::mul(x0, x0), sigma));
-        const bool cancel = !(md::lead(x0) <= 0.0);  // x0 - mu would cancel
-        const R a = cancel ? RN::add(x0, mu) : RN::sub(x0, mu);
-        const bool under = cancel && md::lead(sigma) < __dmul_rn(md::lead(a), pow2(kReflectUnder - E));
-        // sigma + v0^2 = -2 mu v0, so that beta = -v0 / mu: one division
-        // beside the other warp's, none of them waiting for another
-        if (do_inv) inv = cancel ? RN::neg(RN::tr::div(a, sigma)) : RN::tr::div(RN::one(), a);
-        if (do_beta && !under) beta = cancel ? RN::tr::div(sigma, RN::mul(a, mu)) : RN::neg(RN::tr::div(a, mu));
-      }
-    }
-    if ((threadIdx.x & 31) == 0) {
-      if (do_beta) stn_at<RN>(S.misc, 0, beta);
-      if (do_inv) stn_at<N>(S.misc + 2 * N::width, 0, inv);
-    }
-  }
+  reflect_scalars<N, false>(m, col, S.w, S.misc, 0);
   __syncthreads();
+  int E = 0;
+  if (S.misc[4 * N::width] != 0.0) E = reflect_rescaled<N>(m, nc, ld, col, S.w, S.misc);
   const R beta = ldn_at<RN>(S.misc, 0);
   const bool trivial = md::is_zero(beta);
   // v (as the reference leaves it when there is nothing to reflect) and w
@@ -348,7 +370,7 @@ __device__ void block_reflect(int n, long ld, int c, int e, double *Rm, dense_sm
         T v = N::one();
         if (t > 0) {
           v = ldn_at<N>(col, (long)t * ld);
-          if (!trivial) v = N::mul(E != 0 ? mul_pow2(v, down) : v, inv);
+          if (!trivial) v = N::mul(E != 0 ? mul_pow2(v, pow2(-E)) : v, inv);
         }
         stn_at<N>(S.v, t, v);
       } else if (!trivial) {
